@@ -265,6 +265,8 @@ struct AnalysisArgs {
     int nx, ny, M, p, nox, nl_off, nobs;
     float diag, sqrt_m1, tol, c;
     int max_sweeps, write_v;
+    int nl;                   // window half width in sites (n_obs_local)
+    double dloc, covinf;      // Gaspari-Cohn length, inflation beta
 };
 void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s);
 // ---- the Gram on the tcgen05 tensor cores (gram_tc.cu) ----
@@ -283,6 +285,11 @@ void launch_gram_tc(const GramTcParams& G, const float* dY, const float* dyo, co
                     float* Cout, int* err, cudaStream_t s);
 
 void launch_analysis_args(const AnalysisArgs& a, cudaStream_t s);
+
+// ---- the analysis without an eigensolver (letkf_direct.cu): false when no variant serves the
+// configuration (nothing was launched)
+bool launch_analysis_direct_args(const AnalysisArgs& a, cudaStream_t s);
+int direct_prepare();
 
 // ---- kernels (diag_kernels.cu) ----
 void launch_diag(const lbl_ctx* c, const float* mac, int member, double* red, cudaStream_t s);

@@ -1179,7 +1179,7 @@ size_t analysis_smem_bytes(int M, int nobs) {
 // opt in to large dynamic shared memory once per device (not allowed during capture)
 int analysis_prepare() {
     const int lim = 200 * 1024;
-    int rc = 0;
+    int rc = direct_prepare();
     rc |= int(cudaFuncSetAttribute(analysis_kernel<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
@@ -1309,6 +1309,7 @@ void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s) {
 }
 
 void launch_analysis_args(const AnalysisArgs& a, cudaStream_t s) {
+    if (launch_analysis_direct_args(a, s)) return;
     switch (pad_pow2(a.M)) {
         case 4: launch_analysis_args_mp<4>(a, s); break;
         case 8: launch_analysis_args_mp<8>(a, s); break;

@@ -217,6 +217,9 @@ int analysis_noalloc_impl(const lbl_config* cfg, const float* f_in, float* f_out
     a.c = float(c.u_ref) / float(c.cfl);
     a.max_sweeps = c.jacobi_max_sweeps;
     a.write_v = c.compat_stale_v ? 0 : 1;
+    a.nl = nl;
+    a.dloc = dloc;
+    a.covinf = c.letkf_covinf;
     lbl::launch_obs_ensemble_args(a, s);
     lbl::launch_analysis_args(a, s);
     e = cudaGetLastError();
