@@ -124,6 +124,8 @@ struct lbl_ctx {
     // diagnostics scratch
     double* d_red = nullptr;             // reduction scratch (8 doubles)
     float* d_tmp = nullptr;              // nxy*2 floats (truth fields)
+    float* d_acc = nullptr;              // accessors: the fields computed for the host, [4][nxy], behind d_tmp
+    std::vector<float> h_acc;            // and the host copy of small ones
     float* d_dump = nullptr;             // LETKF matrix dump of one chunk (write_mat only)
     std::vector<float> h_dump;
     std::string io_prefix = "io";        // config::prefix (config.h:287) for the matrix dumps
@@ -296,6 +298,9 @@ void launch_diag(const lbl_ctx* c, const float* mac, int member, double* red, cu
 // per-member vorticity [M][nxy] and ensemble statistics [4][nxy] (mean u, mean v,
 // mean vor, std vor) in the reference's FP32 order; *nan |= 1 on a NaN vorticity
 void launch_output_fields(const lbl_ctx* c, const float* mac, float* vor, float* stats, int* nan, cudaStream_t s);
+// the statistics alone, and one member's rho, u, v and vorticity, [4][nxy], for the accessors
+void launch_ens_stats(const lbl_ctx* c, const float* mac, float* stats, cudaStream_t s);
+void launch_member_fields(const lbl_ctx* c, const float* mac, float* out, cudaStream_t s);
 void launch_rmse(const lbl_ctx* c, const float* mac, const float* ut, const float* vt, double* red,
                  cudaStream_t s);
 void launch_rmse_finish(const lbl_ctx* c, double* red, cudaStream_t s);
