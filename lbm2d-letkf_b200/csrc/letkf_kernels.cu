@@ -116,6 +116,35 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     return r;
 }
 
+// Two FP32 multiply-adds (multiplies), PK: in one instruction (sm_100).  Each half rounds as the scalar
+// one, so sums kept in even and odd halves and element-wise updates keep their bits.  The analysis phase,
+// packed against scalar: 512^2 x 64 (the wide kernel) 44.7 / 47.8 ms, 256^2 x 64 13.9 / 15.0, 256^2 x 32 2.27 / 2.33 ms,
+// 160 x 96 x 23 0.78 / 0.81; but 256^2 x 16 0.49 / 0.47 and 64^2 x 8 0.107 / 0.088 ms, where the columns are short
+// and every element also passes through a shuffle: those stay scalar.
+template <bool PK>
+__device__ __forceinline__ void fma_pair(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0, float c1) {
+    if constexpr (PK) {
+        asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n"
+            " fma.rn.f32x2 c, a, b, c;\n mov.b64 {%0, %1}, c;\n}"
+            : "=f"(d0), "=f"(d1)
+            : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+    } else {
+        d0 = fmaf(a0, b0, c0);
+        d1 = fmaf(a1, b1, c1);
+    }
+}
+template <bool PK>
+__device__ __forceinline__ void mul_pair(float& d0, float& d1, float b) {
+    if constexpr (PK) {
+        asm("{\n .reg .b64 a, b;\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %2};\n mul.rn.f32x2 a, a, b;\n mov.b64 {%0, %1}, a;\n}"
+            : "+f"(d0), "+f"(d1)
+            : "f"(b));
+    } else {
+        d0 *= b;
+        d1 *= b;
+    }
+}
+
 template <int MP>
 __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -167,6 +196,7 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
                                                        const int* __restrict__ wcnt, int* __restrict__ stats,
                                                        AnaParams A, DumpPtrs D) {
     constexpr int GPW = 32 / MP;
+    constexpr bool kPacked = MP == 32;  // see fma_pair
     extern __shared__ float smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -289,10 +319,8 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
 #pragma unroll
             for (int l = 0; l < MP; l += 4) {
                 const float4 r4 = *reinterpret_cast<const float4*>(row + l);
-                qv[l + 0] = fmaf(ek, r4.x, qv[l + 0]);
-                qv[l + 1] = fmaf(ek, r4.y, qv[l + 1]);
-                qv[l + 2] = fmaf(ek, r4.z, qv[l + 2]);
-                qv[l + 3] = fmaf(ek, r4.w, qv[l + 3]);
+                fma_pair<kPacked>(qv[l + 0], qv[l + 1], ek, ek, r4.x, r4.y, qv[l + 0], qv[l + 1]);
+                fma_pair<kPacked>(qv[l + 2], qv[l + 3], ek, ek, r4.z, r4.w, qv[l + 2], qv[l + 3]);
             }
         }
 #pragma unroll
@@ -315,10 +343,8 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
 #pragma unroll
                 for (int t = 0; t < MP; t += 4) {
                     const float4 q4 = *reinterpret_cast<const float4*>(sQ + l * MP + t);
-                    av[t + 0] = fmaf(q4.x, vl, av[t + 0]);
-                    av[t + 1] = fmaf(q4.y, vl, av[t + 1]);
-                    av[t + 2] = fmaf(q4.z, vl, av[t + 2]);
-                    av[t + 3] = fmaf(q4.w, vl, av[t + 3]);
+                    fma_pair<kPacked>(av[t + 0], av[t + 1], q4.x, q4.y, vl, vl, av[t + 0], av[t + 1]);
+                    fma_pair<kPacked>(av[t + 2], av[t + 3], q4.z, q4.w, vl, vl, av[t + 2], av[t + 3]);
                 }
             }
             __syncwarp();
@@ -344,11 +370,11 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
         float sc = 1.f;
         for (int sw = 0; sw < A.max_sweeps; sw++) {
 #pragma unroll
-            for (int l = 0; l < MP; l++) qv[l] *= sc;
+            for (int l = 0; l < MP; l += 2) mul_pair<kPacked>(qv[l], qv[l + 1], sc);
             sc = 1.f;
             float a0 = 0.f, a1 = 0.f;
 #pragma unroll
-            for (int l = 0; l < MP; l += 2) { a0 = fmaf(qv[l], qv[l], a0); a1 = fmaf(qv[l + 1], qv[l + 1], a1); }
+            for (int l = 0; l < MP; l += 2) fma_pair<kPacked>(a0, a1, qv[l], qv[l + 1], qv[l], qv[l + 1], a0, a1);
             float a = a0 + a1;
             bool rot = false, wide = false;
             float worst = 0.f;  // largest g^2 / (a b) of the sweep
@@ -362,7 +388,7 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
                 const float sp = __shfl_xor_sync(0xffffffffu, sc, rr);
                 float g0 = 0.f, g1 = 0.f;
 #pragma unroll
-                for (int l = 0; l < MP; l += 2) { g0 = fmaf(qv[l], pq[l], g0); g1 = fmaf(qv[l + 1], pq[l + 1], g1); }
+                for (int l = 0; l < MP; l += 2) fma_pair<kPacked>(g0, g1, qv[l], qv[l + 1], pq[l], pq[l + 1], g0, g1);
                 const float g = (g0 + g1) * (sc * sp);
                 const float b = __shfl_xor_sync(0xffffffffu, a, rr);
                 const bool low = k < (k ^ rr);
@@ -385,7 +411,8 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
                         // low: cs a - sn b; high: sn a + cs b (sn = cs t), with the scales
                         const float rho = (low ? -t : t) * __fdividef(sp, sc);
 #pragma unroll
-                        for (int l = 0; l < MP; l++) qv[l] = fmaf(rho, pq[l], qv[l]);
+                        for (int l = 0; l < MP; l += 2)
+                            fma_pair<kPacked>(qv[l], qv[l + 1], rho, rho, pq[l], pq[l + 1], qv[l], qv[l + 1]);
                         sc *= cs;
                         a = low ? a - t * g : a + t * g;
                     }
@@ -796,10 +823,8 @@ __global__ void __launch_bounds__(kWideThreads, TC ? 4 : 5) analysis_wide_kernel
 #pragma unroll
             for (int l = 0; l < kHalf; l += 4) {
                 const float4 r4 = *reinterpret_cast<const float4*>(row + hx(r0) + l);
-                qv[l + 0] = fmaf(ek, r4.x, qv[l + 0]);
-                qv[l + 1] = fmaf(ek, r4.y, qv[l + 1]);
-                qv[l + 2] = fmaf(ek, r4.z, qv[l + 2]);
-                qv[l + 3] = fmaf(ek, r4.w, qv[l + 3]);
+                fma_pair<true>(qv[l + 0], qv[l + 1], ek, ek, r4.x, r4.y, qv[l + 0], qv[l + 1]);
+                fma_pair<true>(qv[l + 2], qv[l + 3], ek, ek, r4.z, r4.w, qv[l + 2], qv[l + 3]);
             }
         }
         if (!TC) {
@@ -836,10 +861,10 @@ __global__ void __launch_bounds__(kWideThreads, TC ? 4 : 5) analysis_wide_kernel
                 for (int l = 0; l < kHalf; l += 4) {
                     const float4 a4 = *reinterpret_cast<const float4*>(qo + 2 * c * kHS + l);
                     const float4 b4 = *reinterpret_cast<const float4*>(qt + 2 * c * kHS + l);
-                    qv[l + 0] = fmaf(b4.x, vt, fmaf(a4.x, vo, qv[l + 0]));
-                    qv[l + 1] = fmaf(b4.y, vt, fmaf(a4.y, vo, qv[l + 1]));
-                    qv[l + 2] = fmaf(b4.z, vt, fmaf(a4.z, vo, qv[l + 2]));
-                    qv[l + 3] = fmaf(b4.w, vt, fmaf(a4.w, vo, qv[l + 3]));
+                    fma_pair<true>(qv[l + 0], qv[l + 1], a4.x, a4.y, vo, vo, qv[l + 0], qv[l + 1]);
+                    fma_pair<true>(qv[l + 2], qv[l + 3], a4.z, a4.w, vo, vo, qv[l + 2], qv[l + 3]);
+                    fma_pair<true>(qv[l + 0], qv[l + 1], b4.x, b4.y, vt, vt, qv[l + 0], qv[l + 1]);
+                    fma_pair<true>(qv[l + 2], qv[l + 3], b4.z, b4.w, vt, vt, qv[l + 2], qv[l + 3]);
                 }
             }
             __syncthreads();  // sA holds the Jacobi's home slots next
@@ -905,7 +930,7 @@ __global__ void __launch_bounds__(kWideThreads, TC ? 4 : 5) analysis_wide_kernel
                     for (int j = 0; j < H; j++) {
                         float g0 = 0.f, g1 = 0.f;
 #pragma unroll
-                        for (int l = 0; l < 16; l += 2) { g0 = fmaf(xa[l], xb[l], g0); g1 = fmaf(xa[l + 1], xb[l + 1], g1); }
+                        for (int l = 0; l < 16; l += 2) fma_pair<true>(g0, g1, xa[l], xa[l + 1], xb[l], xb[l + 1], g0, g1);
                         const float g = quad_sum(g0 + g1) * (sa * sb);
                         const bool alow = ca < cb;
                         const float alo = alow ? na : nb, ahi = alow ? nb : na;
@@ -929,10 +954,10 @@ __global__ void __launch_bounds__(kWideThreads, TC ? 4 : 5) analysis_wide_kernel
                             const float rlo = -tt * __fdividef(shi, slo), rhi = tt * __fdividef(slo, shi);
                             const float ra = alow ? rlo : rhi, rb = alow ? rhi : rlo;
 #pragma unroll
-                            for (int l = 0; l < 16; l++) {
-                                const float a0 = xa[l];
-                                xa[l] = fmaf(ra, xb[l], a0);
-                                xb[l] = fmaf(rb, a0, xb[l]);
+                            for (int l = 0; l < 16; l += 2) {
+                                const float a0 = xa[l], a1 = xa[l + 1];
+                                fma_pair<true>(xa[l], xa[l + 1], ra, ra, xb[l], xb[l + 1], a0, a1);
+                                fma_pair<true>(xb[l], xb[l + 1], rb, rb, a0, a1, xb[l], xb[l + 1]);
                             }
                             sa *= cs;
                             sb *= cs;
