@@ -262,14 +262,17 @@ struct AnalysisArgs {
     const float* yo;          // [3][nsites] u, v, rho at the sites
     float* dY;                // [3][nsites][M] scratch
     float* dyo;               // [3][nsites] scratch
-    const int* wtab;          // int4 [p*p][nobs] + int [p*p] counts
+    int* wtab;                // int4 [p*p][nobs] + int [p*p] counts, rebuilt by launch_obs_ensemble_args
     int* stats;               // int[4] scratch
     int nx, ny, M, p, nox, nl_off, nobs;
     float diag, sqrt_m1, tol, c;
     int max_sweeps, write_v;
     int nl;                   // window half width in sites (n_obs_local)
     double dloc, covinf;      // Gaspari-Cohn length, inflation beta
+    int off;                  // window offset (obs_offset)
+    double sig_u, sig_rho;    // observation errors
 };
+// the observation operator, the weight table a.wtab and the cleared counters a.stats, in one launch
 void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s);
 // ---- the Gram on the tcgen05 tensor cores (gram_tc.cu) ----
 struct GramTcParams {

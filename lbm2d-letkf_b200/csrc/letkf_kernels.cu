@@ -63,8 +63,8 @@ struct DumpPtrs {
 // H(x) at every observation site for every member, centred on the member mean.
 // One warp per site; lanes stride over members.
 // ---------------------------------------------------------------------------
-__global__ void obs_ensemble_kernel(const float* __restrict__ f, const float* __restrict__ yo,
-                                    float* __restrict__ dY, float* __restrict__ dyo, AnaParams A) {
+__device__ __forceinline__ void obs_site(const float* __restrict__ f, const float* __restrict__ yo,
+                                         float* __restrict__ dY, float* __restrict__ dyo, const AnaParams& A) {
     const int lane = threadIdx.x & 31;
     const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (s >= A.nsites) return;
@@ -106,6 +106,92 @@ __global__ void obs_ensemble_kernel(const float* __restrict__ f, const float* __
         }
         if (lane == 0) dyo[size_t(v) * A.nsites + s] = yo[size_t(v) * A.nsites + s] - mean;
     }
+}
+
+__global__ void obs_ensemble_kernel(const float* __restrict__ f, const float* __restrict__ yo,
+                                    float* __restrict__ dY, float* __restrict__ dyo, AnaParams A) {
+    obs_site(f, yo, dY, dyo, A);
+}
+
+// Gaspari-Cohn weight (letkf.cu:104-109) as IEEE double operations in the source
+// order of the host table builder (lbl_api.cu), so the device-built table below is
+// bit-identical to the one lbl_create uploads: no contraction into FMAs.
+__device__ double gc_weight_rn(double d) {
+    if (d <= 0) return 1.0;
+    const double d2 = __dmul_rn(d, d), d3 = __dmul_rn(d2, d), d4 = __dmul_rn(d3, d), d5 = __dmul_rn(d4, d);
+    const double t3 = __ddiv_rn(__dmul_rn(d3, 5.), 8.), t4 = __ddiv_rn(__dmul_rn(d2, 5.), 3.);
+    if (d <= 1) {
+        const double nd5 = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(-d, d), d), d), d);
+        double s = __dadd_rn(__ddiv_rn(nd5, 4.), __ddiv_rn(d4, 2.));
+        s = __dadd_rn(s, t3);
+        s = __dsub_rn(s, t4);
+        return __dadd_rn(s, 1.);
+    }
+    if (d <= 2) {
+        double s = __dsub_rn(__ddiv_rn(d5, 12.), __ddiv_rn(d4, 2.));
+        s = __dadd_rn(s, t3);
+        s = __dadd_rn(s, t4);
+        s = __dsub_rn(s, __dmul_rn(d, 5.));
+        s = __dadd_rn(s, 4.);
+        return __dsub_rn(s, __ddiv_rn(2. / 3., d));
+    }
+    return 0.0;
+}
+
+// What the allocation-free entry point prepares on every call, in one launch: the first obs_blocks
+// blocks are obs_ensemble_kernel's; the others build the window weight table (set_rR, letkf.cu:75-114), one
+// warp per pattern (i mod p, j mod p): the window slots with weight > 0 in slot order, {slot, var, sqrt(w)
+// bits, w bits}, then the pattern's count at tab[4 p^2 nobs + pattern].  A lane takes a site; a scan
+// over the warp gives its place.  (One thread per pattern in a launch of its own, a memset and then the
+// operator: a call at 128^2 x 4 pointwise 46 against 43 us now, at 160 x 96 x 23 every 2 points 162 / 141, at
+// 256^2 x 16 every 4 points 382 / 352.)
+struct TableJob {
+    int obs_blocks, nl, off;
+    double dloc, sig_u, sig_rho;
+    int *tab, *stats;
+};
+__global__ void obs_table_kernel(const float* __restrict__ f, const float* __restrict__ yo, float* __restrict__ dY,
+                                 float* __restrict__ dyo, AnaParams A, TableJob T) {
+    if (int(blockIdx.x) < T.obs_blocks) {
+        obs_site(f, yo, dY, dyo, A);
+        return;
+    }
+    if (int(blockIdx.x) == T.obs_blocks && threadIdx.x < 4) T.stats[threadIdx.x] = 0;
+    const int lane = threadIdx.x & 31, p = A.p, nox = A.nox, nobs = A.n_pat_max;
+    const int pat = ((int(blockIdx.x) - T.obs_blocks) * int(blockDim.x) + int(threadIdx.x)) >> 5;
+    if (pat >= p * p) return;
+    const int pi = pat % p, pj = pat / p;
+    int n = 0;
+    for (int s0 = 0; s0 < nox * nox; s0 += 32) {
+        const int st = s0 + lane, b = st / nox, a = st - b * nox;
+        const int di = pi - (a - A.nl_off) * p, dj = pj - (b - A.nl_off) * p;
+        float w[3] = {0.f, 0.f, 0.f};
+        int mine = 0;
+        if (st < nox * nox && abs(di) <= T.nl * p && abs(dj) <= T.nl * p) {
+            const double g =
+                p > 1 ? gc_weight_rn(__ddiv_rn(__dsqrt_rn(double(di * di + dj * dj)), __dadd_rn(T.dloc, 1e-6))) : 1.0;
+#pragma unroll
+            for (int var = 0; var < 3; var++) {
+                const double sig = var == 2 ? T.sig_rho : T.sig_u;
+                w[var] = __double2float_rn(__ddiv_rn(g, __dmul_rn(sig, sig)));
+                mine += w[var] > 0.f ? 1 : 0;
+            }
+        }
+        int at = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, at, 31);
+        int4* e = reinterpret_cast<int4*>(T.tab) + size_t(pat) * nobs + n + at - mine;
+#pragma unroll
+        for (int var = 0; var < 3; var++)
+            if (w[var] > 0.f)
+                *e++ = make_int4(a + nox * b + var * nox * nox, var, __float_as_int(__fsqrt_rn(w[var])), __float_as_int(w[var]));
+        n += total;
+    }
+    if (lane == 0) T.tab[size_t(4) * p * p * nobs + pat] = n;
 }
 
 // square root for the Jacobi rotation angle: t only picks the angle, and cs = (1 + t^2)^-1/2
@@ -1329,8 +1415,9 @@ void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s) {
     const AnaParams A = params_from_args(a);
     const int threads = 256;
     const long long total = (long long)A.nsites * 32;
-    const int grid = int((total + threads - 1) / threads);
-    obs_ensemble_kernel<<<grid, threads, 0, s>>>(a.f_in, a.yo, a.dY, a.dyo, A);
+    TableJob T{int((total + threads - 1) / threads), a.nl, a.off, a.dloc, a.sig_u, a.sig_rho, a.wtab, a.stats};
+    const int grid = T.obs_blocks + (a.p * a.p * 32 + threads - 1) / threads;
+    obs_table_kernel<<<grid, threads, 0, s>>>(a.f_in, a.yo, a.dY, a.dyo, A, T);
 }
 
 void launch_analysis_args(const AnalysisArgs& a, cudaStream_t s) {
