@@ -260,7 +260,7 @@ int lbl_event_elapsed(lbl_ctx* ctx, int slot_a, int slot_b, double* ms);
  * device then holds it until exit.  The first call on a device also looks the
  * array up (cudaGetSymbolAddress) and must come before any stream capture.  All
  * calls share the array: calls that overlap on the GPU race and must be
- * serialised.  Every call only enqueues kernels and a memset on `stream` (a
+ * serialised.  Every call only enqueues kernels on `stream` (a
  * cudaStream_t, NULL = legacy default stream): the window weight table is rebuilt
  * on the device and the counters cleared each time, with no host memory involved.
  * host_stats (int[4]: max sweeps, non-converged points, NaN flag, sweep total) is
