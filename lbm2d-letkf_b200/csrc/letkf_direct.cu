@@ -163,6 +163,7 @@ struct Rows {
     int row0;               // matrix row of slot 0 (2^20 when it is none: never a pivot)
     bool carry;             // slot 1 holds a carried row
     bool last0;             // one of the last two matrix rows
+    bool entry;             // the lane has an entry of whole-row reflections
     // offsets into the CTA's shared memory:
     int px0;                // sx + row, less k0 (moves down two per pair)
     int pR;                 // R' entry of the carried row, [column][12]
@@ -228,7 +229,8 @@ __device__ __forceinline__ void reflect(u64 (&r)[2][N / 2], Rows& R, const int k
         if (below0 && R.row0 < R.n) smem[R.pV0] = vr0;
         R.pV0 += R.n - 2 - k;
     } else {                // whole rows, zero at and above the pivot
-        smem[R.pV0] = vr0;
+        // (at order 8 sixteen lanes hold a point: the eight without an entry would store zeros over the others')
+        if (N == 16 || R.entry) smem[R.pV0] = vr0;
         R.pV0 += N;
     }
     __syncwarp();
@@ -614,6 +616,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
         R.row0 = mat0 ? lane : 1 << 20;  // a lane without a row is never a pivot and writes beside the arrays
         R.carry = carry;
         R.last0 = mat0 && lane >= n - 2;
+        R.entry = lane < N;
         const int at = int(base - smem);
         R.px0 = at + N + (mat0 ? lane : N + lane % N);
         R.pT = at + 6 * N;
