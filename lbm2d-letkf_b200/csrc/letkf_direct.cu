@@ -421,18 +421,23 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
 #pragma unroll
                 for (int q = 0; q < kQ; q++) d[q] -= sum[q];
             }
-            // the point's observations, (slot, scaled weight); the rows past them take the first one's slot
-            // with weight 0: rows of the identity
+            // the point's observations, (slot, scaled weight).  The rows past them are rows of the identity, zeros
+            // whatever the window holds (their slot is the block's first, never multiplied); a pattern whose
+            // weights all round to zero has only such rows, and no table entry to read
 #pragma unroll 1
             for (int e = lane; e < N; e += LPP) {
-                const int4 w = __ldg(ent + (e < cnt ? e : 0));
-                *reinterpret_cast<float2*>(sS + 2 * e) =
-                    make_float2(__int_as_float(sOff[w.x] + blk), e < cnt ? __int_as_float(w.z) * A.inv_sqrt_a : 0.f);
+                float2 ow = make_float2(__int_as_float(blk), 0.f);
+                if (e < cnt) {
+                    const int4 w = __ldg(ent + e);
+                    ow = make_float2(__int_as_float(sOff[w.x] + blk), __int_as_float(w.z) * A.inv_sqrt_a);
+                }
+                *reinterpret_cast<float2*>(sS + 2 * e) = ow;
             }
             __syncwarp();
             // rows R = dX C^T (and g = d): lane = observation, then to the carried rows' lanes
             u64 acc[5];
             const int o1 = min(lane, N - 1);
+            const bool observed = o1 < cnt;
             const float sw = sS[2 * o1 + 1];
             const float* yrow = sY + __float_as_int(sS[2 * o1]) * ms;
 #pragma unroll
@@ -441,7 +446,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
             for (int m = 0; m < mx; m += 4) {
                 // the weighted window by members, for the products and the update
                 float4 y = *reinterpret_cast<const float4*>(yrow + m);
-                y.x *= sw; y.y *= sw; y.z *= sw; y.w *= sw;
+                y = observed ? make_float4(y.x * sw, y.y * sw, y.z * sw, y.w * sw) : make_float4(0.f, 0.f, 0.f, 0.f);
                 if (lane < N) {
                     sC[(m + 0) * N + lane] = y.x;
                     sC[(m + 1) * N + lane] = y.y;
@@ -470,7 +475,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
                     rows[(2 * q + 1) * N + lane] = hi_of(acc[q]);
                 }
                 rows[8 * N + lane] = lo_of(acc[4]);
-                rows[9 * N + lane] = sw * sDyo[__float_as_int(sS[2 * o1])];
+                rows[9 * N + lane] = observed ? sw * sDyo[__float_as_int(sS[2 * o1])] : 0.f;
             }
             __syncwarp();
             if (carry)
