@@ -511,14 +511,15 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
                 for (int q = 0; q < kQ; q++)
                     sX[q * N + lane] = lane < M ? __ldg(A.fin + (size_t(lane) * kQ + q) * A.nxy + point) : 0.f;
             // Gram: row `lane` of C^T C, and g = C^T d (letkf_solver.h:252-254)
-            const float inv_a = A.inv_sqrt_a * A.inv_sqrt_a;
             {
                 // On the tensor cores, the whole warp for one point after the other, eight observations at a
-                // time: lane (g, c) brings members g, g + 8, ... of observations c and c + 4, which are both
-                // its share of A = (w dY)^T and of B = dY.  Every operand is split into two TF32 terms, three
-                // MMAs per tile with FP32 sums (about 2^-22 relative).  The same products by multiply-adds read
-                // the window row of every observation in every lane: half of the shared-memory traffic of a point
-                // at 16 members, and five times the instructions.
+                // time: lane (g, c) brings members g, g + 8, ... of observations c and c + 4 of C, which are both
+                // its share of A = C^T and of B.  Every entry is split into two TF32 terms (2^-23 relative) and all
+                // four products are summed in FP32, the smallest first.  As (w dY)^T dY, whose factors are rounded and
+                // split apart, in three products, the error against FP64 was 1.3 to 2 times as large (64 x 32 points of 16 and
+                // 32 members, 27 and 42 observations, kappa 1e3 to 1e6) and above the Jacobi kernel's from kappa 1e3 on.
+                // Now it is that of multiply-adds, which read the window row of every observation in every lane: 390 against
+                // 348 us at 256^2 x 16 (42 observations), 1708 / 1674 at 256^2 x 32.
                 constexpr int MT = N / 16, YT = N / 8;
                 const int g8 = wl >> 2, c4 = wl & 3;
 #pragma unroll 1
@@ -534,29 +535,29 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
                     for (int i2 = 0; i2 < YT; i2++) gs[i2] = 0.f;
 #pragma unroll 1
                     for (int o0 = 0; o0 < pcnt; o0 += 8) {
-                        uint32_t ah[2][YT], al[2][YT], bh[2][YT], bl[2][YT];
+                        uint32_t bh[2][YT], bl[2][YT];
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
                             const int o = o0 + c4 + 4 * h;  // past the end: the first observation with weight 0
                             const int4 e = __ldg(pent + (o < pcnt ? o : 0));
                             const int slot = sOff[e.x] + pblk;
-                            const float w = o < pcnt ? __int_as_float(e.w) * inv_a : 0.f;
-                            const float d = sDyo[slot];
+                            const float sw = o < pcnt ? __int_as_float(e.z) * A.inv_sqrt_a : 0.f;
+                            const float d = sw * sDyo[slot];
 #pragma unroll
                             for (int i2 = 0; i2 < YT; i2++) {
-                                const float y = sY[slot * ms + g8 + 8 * i2], wy = w * y;
+                                const float y = sw * sY[slot * ms + g8 + 8 * i2];
                                 split_tf32(y, bh[h][i2], bl[h][i2]);
-                                split_tf32(wy, ah[h][i2], al[h][i2]);
-                                gs[i2] = fmaf(wy, d, gs[i2]);
+                                gs[i2] = fmaf(y, d, gs[i2]);
                             }
                         }
 #pragma unroll
                         for (int i1 = 0; i1 < MT; i1++)
 #pragma unroll
                             for (int i2 = 0; i2 < YT; i2++) {
-                                mma_tf32(acc[i1][i2], ah[0][2 * i1], ah[0][2 * i1 + 1], ah[1][2 * i1], ah[1][2 * i1 + 1], bh[0][i2], bh[1][i2]);
-                                mma_tf32(acc[i1][i2], ah[0][2 * i1], ah[0][2 * i1 + 1], ah[1][2 * i1], ah[1][2 * i1 + 1], bl[0][i2], bl[1][i2]);
-                                mma_tf32(acc[i1][i2], al[0][2 * i1], al[0][2 * i1 + 1], al[1][2 * i1], al[1][2 * i1 + 1], bh[0][i2], bh[1][i2]);
+                                mma_tf32(acc[i1][i2], bl[0][2 * i1], bl[0][2 * i1 + 1], bl[1][2 * i1], bl[1][2 * i1 + 1], bl[0][i2], bl[1][i2]);
+                                mma_tf32(acc[i1][i2], bl[0][2 * i1], bl[0][2 * i1 + 1], bl[1][2 * i1], bl[1][2 * i1 + 1], bh[0][i2], bh[1][i2]);
+                                mma_tf32(acc[i1][i2], bh[0][2 * i1], bh[0][2 * i1 + 1], bh[1][2 * i1], bh[1][2 * i1 + 1], bl[0][i2], bl[1][i2]);
+                                mma_tf32(acc[i1][i2], bh[0][2 * i1], bh[0][2 * i1 + 1], bh[1][2 * i1], bh[1][2 * i1 + 1], bh[0][i2], bh[1][i2]);
                             }
                     }
                     float* pbase = base + (pg - grp) * (region_floats(S::FIXED, N, DUAL, mx));
