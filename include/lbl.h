@@ -267,8 +267,9 @@ int lbl_event_elapsed(lbl_ctx* ctx, int slot_a, int slot_b, double* ms);
  * optional; given, the call waits for the stream and returns LBL_ERR_NAN on a NaN
  * in the analysis.  Without it the call does not wait and cannot report a NaN.  Nine or
  * more members are solved without an eigensolver (one sweep per point, never
- * non-converged, whatever jacobi_tol and jacobi_max_sweeps ask); the analysis then
- * agrees with lbl_assimilate's to about 1e-5 of an increment.
+ * non-converged), but for points whose matrix is ill-conditioned (the observations
+ * pull more than about 1e4 times as hard as the inflated background), which the
+ * Jacobi iteration solves.
  * err (optional) receives a message of at most err_cap bytes. */
 int lbl_letkf_analysis_noalloc(const lbl_config* cfg, const float* f_in, float* f_out, float* mac_out,
                                const float* yo_sites, void* stream, int* host_stats, char* err, size_t err_cap);

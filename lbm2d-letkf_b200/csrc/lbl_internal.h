@@ -263,7 +263,7 @@ struct AnalysisArgs {
     float* dY;                // [3][nsites][M] scratch
     float* dyo;               // [3][nsites] scratch
     int* wtab;                // int4 [p*p][nobs] + int [p*p] counts, rebuilt by launch_obs_ensemble_args
-    int* stats;               // int[4] scratch
+    int* stats;               // int[5] scratch: the four counters, then 1 when the direct solver left a point
     int nx, ny, M, p, nox, nl_off, nobs;
     float diag, sqrt_m1, tol, c;
     int max_sweeps, write_v;
@@ -291,9 +291,14 @@ void launch_gram_tc(const GramTcParams& G, const float* dY, const float* dyo, co
 
 void launch_analysis_args(const AnalysisArgs& a, cudaStream_t s);
 
-// ---- the analysis without an eigensolver (letkf_direct.cu): false when no variant serves the
-// configuration (nothing was launched)
-bool launch_analysis_direct_args(const AnalysisArgs& a, cudaStream_t s);
+// ---- the analysis without an eigensolver (letkf_direct.cu).  What it was launched for: no point (no variant
+// serves the configuration, nothing was launched), every point, or every point but those whose matrix is
+// too ill-conditioned for it, which it marks with kLeftPoint and counts on the Jacobi kernel to solve
+enum class Direct { kNone, kAll, kLeavesSome };
+Direct launch_analysis_direct_args(const AnalysisArgs& a, cudaStream_t s);
+// the mark, in place of the first member's density: a NaN pattern that no arithmetic gives (NVIDIA's
+// arithmetic returns 0x7fffffff)
+constexpr unsigned kLeftPoint = 0xffa5c35au;
 int direct_prepare();
 
 // ---- kernels (diag_kernels.cu) ----

@@ -18,7 +18,7 @@
 //      a matrix row and a carried row per lane in registers, and each step needs two small broadcasts
 //      through shared memory, the pivot column and B v.
 //   2. T^-1/2 as a sum of N shifted inverses, t^-1/2 = sum_j w_j / (t + s_j) on [1, kappa]:
-//      Zolotarev's best rational approximation (relative error below 2e-8 up to kappa = 1e6;
+//      Zolotarev's best rational approximation (relative error below 2e-8 up to kappa = 1e12;
 //      shifts from Jacobi elliptic functions, computed on the host).  kappa is bounded
 //      per point by Gershgorin's circles of T, and picks one of the tables at powers of 4.
 //      Every shifted T is solved by one tridiagonal elimination; T^-1 g' likewise.
@@ -28,7 +28,9 @@
 //              t^-1/2: the same shifts, weights -w_j / (1 + s_j), no cancellation;
 //      s = R' T^-1 g', the update of the mean.
 // A point costs 4/3 n^3 + O(n^2) operations against 9 n^3 per Jacobi sweep, and has no
-// iteration to converge: the caller's sweep limit and tolerance are met by any value.
+// iteration to converge.  In FP32 the reduction keeps the small eigenvalues less well than the iteration
+// on columns does: a tile with a point above the limit of its form (trace_limit) is marked and left to
+// the Jacobi kernel, launched behind this one.
 #include <algorithm>
 #include <cmath>
 
@@ -105,8 +107,9 @@ __device__ __forceinline__ float mean_of(float s, float m, float inv_m) {
 }
 
 constexpr int kB = 10;          // carried rows: nine of R, then g
-constexpr int kMaxPoles = 20;   // shifts of one table
-constexpr int kTables = 12;     // kappa <= 4^1 .. 4^12
+constexpr int kMaxPoles = 30;   // shifts of one table
+constexpr int kTables = 20;     // kappa <= 4^1 .. 4^20
+constexpr float kKappaMax = 1e8f;  // a point of order 16 above it counts as not converged: its mean update is good to 1e-3
 
 // the shifts and weights, one table per kappa = 4^(b+1)
 struct PoleTables {
@@ -126,6 +129,7 @@ struct DirParams {
     int ms;                 // floats per slot of the staged window (at least N in the primal form): 4 (mod 8),
                             // so that eight lanes reading 16 bytes of consecutive slots hit different banks
     float inv_sqrt_a, sqrt_beta, c, inv_m;
+    float limit;            // the largest bound of a tile's traces of C^T C solved here
     int write_v;
 };
 
@@ -296,6 +300,7 @@ template <int N, int LPP, bool DUAL>
 __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_direct_kernel(const DirParams A, const __grid_constant__ PoleTables T) {
     using S = Shape<N, LPP, DUAL>;
     constexpr int kWarps = warps_of(N);
+    constexpr bool LIMITED = !DUAL;  // see trace_limit
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, wl = tid & 31, warp = tid >> 5;
     const int lane = wl % LPP, grp = wl / LPP;
@@ -315,6 +320,11 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
         const int n2 = A.nox * A.nox, var = o / n2, ab = o - var * n2, b = ab / A.nox, a = ab - b * A.nox;
         sOff[o] = a + ux * b + var * us;
     }
+    int top[3] = {0, 0, 0};  // the lane's member: the largest dY^2 of each variable
+    if constexpr (LIMITED) {
+        if (tid < 96) region[tid] = 0.f;
+        __syncthreads();
+    }
 #pragma unroll 2
     for (int sl = warp; sl < slots; sl += kWarps) {
         const int var = sl / us, s2 = sl - var * us, b = s2 / ux, a = s2 - b * ux;
@@ -323,10 +333,45 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
         si += si < 0 ? A.nsx : 0;
         const size_t site = size_t(var) * A.nsites + si + size_t(A.nsx) * sj;
 #pragma unroll 1
-        for (int m = wl; m < ms; m += 32) sY[sl * ms + m] = m < M ? __ldg(A.dY + site * M + m) : 0.f;
+        for (int m = wl; m < ms; m += 32) {
+            const float y = m < M ? __ldg(A.dY + site * M + m) : 0.f;
+            sY[sl * ms + m] = y;
+            if (LIMITED && m < 32) {  // (a NaN stays one: its square, as an integer, is above every number's)
+                const int y2 = __float_as_int(y * y);
+                top[0] = var == 0 ? max(top[0], y2) : top[0];
+                top[1] = var == 1 ? max(top[1], y2) : top[1];
+                top[2] = var == 2 ? max(top[2], y2) : top[2];
+            }
+        }
         if (wl == 0) sDyo[sl] = __ldg(A.dyo + site);
     }
+    if constexpr (LIMITED) {
+#pragma unroll
+        for (int var = 0; var < 3; var++) atomicMax(reinterpret_cast<int*>(region) + 32 * var + wl, top[var]);
+    }
     __syncthreads();
+    const int tw = A.nbx * A.p, npts = tw * A.nby * A.p;
+    const int rounds = (npts + kWarps * S::GPW - 1) / (kWarps * S::GPW);
+    // ---- a tile that may hold a point above the limit is left to the Jacobi kernel, before it costs a solve.
+    // The trace of C^T C, sum of w |dY|^2 / a, is at least kappa - 1; every member's largest dY of the window
+    // and the weights of the pattern (0, 0) bound it to within a factor of a few.
+    if constexpr (LIMITED) {
+        float t = 0.f;
+#pragma unroll
+        for (int var = 0; var < 3; var++) t = fmaf(__int_as_float(__ldg(A.stats + 5 + var)), region[32 * var + wl], t);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (!(t * (A.inv_sqrt_a * A.inv_sqrt_a) <= A.limit)) {  // (all warps see the same sum)
+#pragma unroll 1
+            for (int pt = tid; pt < npts; pt += 32 * kWarps) {
+                const int i = bx0 * A.p + pt % tw, j = by0 * A.p + pt / tw;
+                if (i < A.nx && j < A.ny) A.mac[i + A.nx * j] = __uint_as_float(kLeftPoint);
+            }
+            if (tid == 0) A.stats[4] = 1;
+            return;
+        }
+        __syncthreads();  // the region is the points' from here on
+    }
     // ---- the point's shared region
     constexpr int VSTRIDE = LPP == 32 ? 0 : N;
     float* base = region + size_t(warp * S::GPW + grp) *
@@ -344,9 +389,8 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
     float* sX = sS + 2 * N;        // DUAL: dX [mx][12]; else the rows on their way in: [12][N]
     float* sC = sX + 12 * mx;      // DUAL: C [mx][N]
 
-    const int tw = A.nbx * A.p, npts = tw * A.nby * A.p;
     bool bad = false;
-    const int rounds = (npts + kWarps * S::GPW - 1) / (kWarps * S::GPW);
+    int noconv = 0;
 #pragma unroll 1
     for (int round = 0; round < rounds; round++) {
         __syncthreads();  // the stages' barriers keep the warps on the same instructions
@@ -655,6 +699,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
         int tab = 0;
         for (float lim = 4.f; tab < kTables - 1 && kap > lim; lim *= 4.f) tab++;
         const int np = T.n[tab];
+        if (DUAL && N > 8 && active && lane == 0) noconv += kap <= kKappaMax ? 0 : 1;
 
         if constexpr (LPP == 16) {
             // lane = (shift j of 8, half h of the carried rows); the eighth shift is 0, for g alone
@@ -904,6 +949,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
         }
     }
     if (bad) atomicOr(A.stats + 2, 1);
+    if (noconv) atomicAdd(A.stats + 1, noconv);
     if (tid == 0) {  // one direct solve per point, counted as one sweep
         const int w = max(0, min(tw, A.nx - bx0 * A.p)), h = max(0, min(A.nby * A.p, A.ny - by0 * A.p));
         atomicMax(A.stats + 0, 1);
@@ -1001,6 +1047,17 @@ const Variant kVariants[] = {
     {16, 16, true, (const void*)analysis_direct_kernel<16, 16, true>},
 };
 
+// The largest bound of a tile's traces of C^T C that the primal form solves; a tile with a larger one goes to the
+// Jacobi kernel.  Rms error against FP64, of an increment, this kernel / the Jacobi kernel (64 x 32 points, an exact
+// operator, by the largest trace):
+//   primal  1e3: 16 members 1.3e-7 / 3.5e-7, 32 1.1e-7 / 5.6e-7; 1.4e4 (27 observations): 16 members 3.8e-7 / 3.2e-7,
+//           32 1.4e-6 / 1.3e-6; 1.5e6: 6.0e-7 / 3.8e-7, 7.3e-5 / 2.9e-5; 1.5e8: 24 members 2.6e-1 / 1.2e-2
+//   dual    order 16, 32 members: 1e3 1.4e-8 / 2.9e-7, 1.6e5 1e-7 / 3.9e-4, 1e7 5e-6 / 5e-3, 1.6e8 2e-4 / 0.14, 6e8 5e-3 /
+//           2e4 (not converged); order 8: 1.8e-8 up to 6e11: no limit
+// The reduction keeps an eigenvalue to 2^-24 of the largest; in the member space, one of every window's is the
+// smallest possible (the members' sum), in the observation space hardly any is.
+float trace_limit(bool dual) { return dual ? INFINITY : 3e4f; }
+
 template <int N, int LPP, bool DUAL>
 int region_of(int mx) {
     using S = Shape<N, LPP, DUAL>;
@@ -1089,10 +1146,10 @@ int direct_prepare() {
     return rc;
 }
 
-bool launch_analysis_direct_args(const AnalysisArgs& g, cudaStream_t s) {
+Direct launch_analysis_direct_args(const AnalysisArgs& g, cudaStream_t s) {
     const int nsx = g.nx / g.p, nsy = g.ny / g.p;
     const Plan P = make_plan(g.M, g.p, g.nox, g.nl_off, g.nl, g.dloc, nsx, nsy);
-    if (P.variant < 0) return false;
+    if (P.variant < 0) return Direct::kNone;
     DirParams A{};
     A.fin = g.f_in; A.fout = g.f_out; A.mac = g.mac_out; A.dY = g.dY; A.dyo = g.dyo;
     A.wtab = reinterpret_cast<const int4*>(g.wtab);
@@ -1106,8 +1163,10 @@ bool launch_analysis_direct_args(const AnalysisArgs& g, cudaStream_t s) {
     A.c = g.c;
     A.inv_m = 1.f / float(A.M);
     A.write_v = g.write_v;
+    const Variant& V = kVariants[P.variant];
+    A.limit = trace_limit(V.dual);
     launch(P, A, s);
-    return true;
+    return std::isinf(A.limit) ? Direct::kAll : Direct::kLeavesSome;
 }
 
 }  // namespace lbl

@@ -21,6 +21,7 @@
 //                        Xa = xbar + dX V (sqrt(M-1) Lambda^-1/2 V^T + Lambda^-1 V^T dY^T R^-1 dyo 1^T)
 //                        written straight into the member-major populations, plus
 //                        the lbm2euler macros (letkf.cu:336-357).
+#include <algorithm>
 #include <cmath>
 
 #include "lbl_internal.h"
@@ -156,12 +157,13 @@ __global__ void obs_table_kernel(const float* __restrict__ f, const float* __res
         obs_site(f, yo, dY, dyo, A);
         return;
     }
-    if (int(blockIdx.x) == T.obs_blocks && threadIdx.x < 4) T.stats[threadIdx.x] = 0;
+    if (int(blockIdx.x) == T.obs_blocks && threadIdx.x < 5) T.stats[threadIdx.x] = 0;
     const int lane = threadIdx.x & 31, p = A.p, nox = A.nox, nobs = A.n_pat_max;
     const int pat = ((int(blockIdx.x) - T.obs_blocks) * int(blockDim.x) + int(threadIdx.x)) >> 5;
     if (pat >= p * p) return;
     const int pi = pat % p, pj = pat / p;
     int n = 0;
+    float sum[3] = {0.f, 0.f, 0.f};
     for (int s0 = 0; s0 < nox * nox; s0 += 32) {
         const int st = s0 + lane, b = st / nox, a = st - b * nox;
         const int di = pi - (a - A.nl_off) * p, dj = pj - (b - A.nl_off) * p;
@@ -175,6 +177,7 @@ __global__ void obs_table_kernel(const float* __restrict__ f, const float* __res
                 const double sig = var == 2 ? T.sig_rho : T.sig_u;
                 w[var] = __double2float_rn(__ddiv_rn(g, __dmul_rn(sig, sig)));
                 mine += w[var] > 0.f ? 1 : 0;
+                sum[var] += w[var];
             }
         }
         int at = mine;
@@ -192,6 +195,13 @@ __global__ void obs_table_kernel(const float* __restrict__ f, const float* __res
         n += total;
     }
     if (lane == 0) T.tab[size_t(4) * p * p * nobs + pat] = n;
+    if (pat == 0)  // the weights of each variable, for the direct solver's choice of points
+#pragma unroll
+        for (int var = 0; var < 3; var++) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum[var] += __shfl_xor_sync(0xffffffffu, sum[var], o);
+            if (lane == 0) T.stats[5 + var] = __float_as_int(sum[var]);
+        }
 }
 
 // square root for the Jacobi rotation angle: t only picks the angle, and cs = (1 + t^2)^-1/2
@@ -274,13 +284,14 @@ constexpr int kWCW = 4, kWCH = 8;
 
 // DUMP = true recomputes the tiles that cover the rows of D and, instead of writing
 // the analysis, writes every intermediate matrix of those rows (need_save_mat).
-template <int MP, bool DUMP>
-__global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__ fin, float* __restrict__ fout,
-                                                       float* __restrict__ mac, const float* __restrict__ dY,
-                                                       const float* __restrict__ dyo,
-                                                       const int4* __restrict__ wtab,
-                                                       const int* __restrict__ wcnt, int* __restrict__ stats,
-                                                       AnaParams A, DumpPtrs D) {
+// LEFT = true solves only the points that the direct kernel left (kLeftPoint in their first member's density).
+// `block` numbers the CTAs of the whole grid.
+template <int MP, bool DUMP, bool LEFT>
+__device__ __forceinline__ void analysis_block(const int block, const float* __restrict__ fin, float* __restrict__ fout,
+                                               float* __restrict__ mac, const float* __restrict__ dY,
+                                               const float* __restrict__ dyo, const int4* __restrict__ wtab,
+                                               const int* __restrict__ wcnt, int* __restrict__ stats,
+                                               const AnaParams& A, const DumpPtrs& D) {
     constexpr int GPW = 32 / MP;
     constexpr bool kPacked = MP == 32;  // see fma_pair
     extern __shared__ float smem[];
@@ -308,7 +319,7 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
     float* sXbar = sY + MP;                    // [9]      ensemble mean (12 reserved)
 
     const int tiles_x = (A.nx + kCW - 1) / kCW;
-    const int tile = (blockIdx.x * (blockDim.x >> 5) + warp) * GPW + grp;
+    const int tile = (block * int(blockDim.x >> 5) + warp) * GPW + grp;
     const int x0 = (tile % tiles_x) * kCW;
     const int y0 = (A.tile_y0 + tile / tiles_x) * kCH;
     const unsigned gmask = (MP == 32) ? 0xffffffffu : (((1u << MP) - 1u) << gbase);
@@ -324,8 +335,12 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
         const int r = idx / kCW;
         const int cc = (r & 1) ? (kCW - 1 - idx % kCW) : (idx % kCW);
         const int i = x0 + cc, j = y0 + r;
-        const bool active = (i < A.nx) && (j < A.ny);  // uniform within the group
+        bool active = (i < A.nx) && (j < A.ny);  // uniform within the group
         const int point = active ? i + A.nx * j : 0;
+        if (LEFT) {
+            active = active && __float_as_uint(__ldcg(mac + point)) == kLeftPoint;
+            if (!__any_sync(0xffffffffu, active)) continue;
+        }
         const bool real_m = active && real_k;
         const bool dump = DUMP && active && j >= D.j0 && j < D.j1;
         const size_t b = dump ? size_t(point - D.point0) : 0;
@@ -647,6 +662,31 @@ __global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__
         if (noconv) atomicAdd(stats + 1, noconv);
         atomicAdd(stats + 3, total_sweeps);
     }
+}
+
+template <int MP, bool DUMP>
+__global__ void __launch_bounds__(128) analysis_kernel(const float* __restrict__ fin, float* __restrict__ fout,
+                                                       float* __restrict__ mac, const float* __restrict__ dY,
+                                                       const float* __restrict__ dyo,
+                                                       const int4* __restrict__ wtab,
+                                                       const int* __restrict__ wcnt, int* __restrict__ stats,
+                                                       AnaParams A, DumpPtrs D) {
+    analysis_block<MP, DUMP, false>(blockIdx.x, fin, fout, mac, dY, dyo, wtab, wcnt, stats, A, D);
+}
+
+// The points that the direct kernel left, on a grid no larger than the GPU: most calls have none (stats[4]),
+// and leave again at once.
+template <int MP>
+__global__ void __launch_bounds__(128) analysis_left_kernel(const float* __restrict__ fin, float* __restrict__ fout,
+                                                            float* __restrict__ mac, const float* __restrict__ dY,
+                                                            const float* __restrict__ dyo,
+                                                            const int4* __restrict__ wtab,
+                                                            const int* __restrict__ wcnt, int* __restrict__ stats,
+                                                            int blocks, AnaParams A) {
+    if (stats[4] == 0) return;
+#pragma unroll 1
+    for (int block = blockIdx.x; block < blocks; block += gridDim.x)
+        analysis_block<MP, false, true>(block, fin, fout, mac, dY, dyo, wtab, wcnt, stats, A, DumpPtrs{});
 }
 
 // ---------------------------------------------------------------------------
@@ -1295,6 +1335,8 @@ int analysis_prepare() {
     rc |= int(cudaFuncSetAttribute(analysis_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    rc |= int(cudaFuncSetAttribute(analysis_left_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    rc |= int(cudaFuncSetAttribute(analysis_left_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
@@ -1395,8 +1437,11 @@ AnaParams params_from_args(const AnalysisArgs& a) {
     return A;
 }
 
+// CTAs of the launch behind the direct kernel: two rounds of the 148 SMs at the one to two that fit
+constexpr int kLeftGrid = 4 * 148;
+
 template <int MP>
-void launch_analysis_args_mp(const AnalysisArgs& a, cudaStream_t s) {
+void launch_analysis_args_mp(const AnalysisArgs& a, bool left, cudaStream_t s) {
     const AnaParams A = params_from_args(a);
     constexpr int GPW = 32 / MP;
     const int warps = 4;
@@ -1404,10 +1449,16 @@ void launch_analysis_args_mp(const AnalysisArgs& a, cudaStream_t s) {
     const size_t sm = analysis_smem_bytes(A.M, A.n_pat_max);
     const int tiles = ((A.nx + kCW - 1) / kCW) * ((A.ny + kCH - 1) / kCH);
     const int grid = (tiles + groups_per_cta - 1) / groups_per_cta;
-    analysis_kernel<MP, false><<<grid, warps * 32, sm, s>>>(a.f_in, a.f_out, a.mac_out, a.dY, a.dyo,
-                                                             reinterpret_cast<const int4*>(a.wtab),
-                                                             a.wtab + size_t(4) * a.p * a.p * a.nobs, a.stats, A,
-                                                             DumpPtrs{});
+    const int4* tab = reinterpret_cast<const int4*>(a.wtab);
+    const int* cnt = a.wtab + size_t(4) * a.p * a.p * a.nobs;
+    if constexpr (MP >= 16)
+        if (left) {
+            analysis_left_kernel<MP><<<std::min(grid, kLeftGrid), warps * 32, sm, s>>>(
+                a.f_in, a.f_out, a.mac_out, a.dY, a.dyo, tab, cnt, a.stats, grid, A);
+            return;
+        }
+    analysis_kernel<MP, false><<<grid, warps * 32, sm, s>>>(a.f_in, a.f_out, a.mac_out, a.dY, a.dyo, tab, cnt,
+                                                            a.stats, A, DumpPtrs{});
 }
 }  // namespace
 
@@ -1421,12 +1472,19 @@ void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s) {
 }
 
 void launch_analysis_args(const AnalysisArgs& a, cudaStream_t s) {
-    if (launch_analysis_direct_args(a, s)) return;
+    switch (launch_analysis_direct_args(a, s)) {
+        case Direct::kAll: return;
+        case Direct::kLeavesSome:  // the points it left, at the iteration's accuracy
+            if (a.M <= 16) launch_analysis_args_mp<16>(a, true, s);
+            else launch_analysis_args_mp<32>(a, true, s);
+            return;
+        case Direct::kNone: break;
+    }
     switch (pad_pow2(a.M)) {
-        case 4: launch_analysis_args_mp<4>(a, s); break;
-        case 8: launch_analysis_args_mp<8>(a, s); break;
-        case 16: launch_analysis_args_mp<16>(a, s); break;
-        case 32: launch_analysis_args_mp<32>(a, s); break;
+        case 4: launch_analysis_args_mp<4>(a, false, s); break;
+        case 8: launch_analysis_args_mp<8>(a, false, s); break;
+        case 16: launch_analysis_args_mp<16>(a, false, s); break;
+        case 32: launch_analysis_args_mp<32>(a, false, s); break;
         default: break;
     }
 }

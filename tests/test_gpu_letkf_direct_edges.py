@@ -1,9 +1,13 @@
 """Edges of the analysis without an eigensolver (csrc/letkf_direct.cu) through the allocation-free
-entry point: windows whose observations weigh nothing."""
+entry point: windows whose observations weigh nothing, and tiles left to the Jacobi kernel."""
+import ctypes
+
 import numpy as np
 import pytest
 
+import lbl
 from test_gpu_letkf_direct import _analyse, _case
+from test_gpu_letkf_direct_precision import _exact_case
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -31,3 +35,41 @@ def test_observations_without_weight_leave_the_inflated_ensemble(M, p, L, sigma)
     want = F.mean(0) + np.sqrt(1.1) * dX
     assert np.max(np.abs(dX)) > 1e-6
     assert np.max(np.abs(got - want)) < 3e-7 * np.max(np.abs(F)) + 4e-6 * np.max(np.abs(dX))
+
+
+def _call(cfg, d_in, d_out, d_mac, d_yo):
+    stats = (ctypes.c_int * 4)()
+    rc = lbl.load_library().lbl_letkf_analysis_noalloc(ctypes.byref(cfg), d_in.data_ptr(), d_out.data_ptr(),
+                                                       d_mac.data_ptr(), d_yo.data_ptr(),
+                                                       torch.cuda.current_stream().cuda_stream, stats, None, 0)
+    return rc, list(stats)
+
+
+@pytest.mark.parametrize("M", [16, 32])
+def test_points_left_to_the_iteration(M):
+    """Half of the grid has a spread of a hundred times the observation error and half a
+    thousandth of that: some tiles are left to the Jacobi kernel.  No mark stays in the moments, which are
+    those of the populations, every point is counted, an analysis in place is the same, and so
+    is a second call."""
+    nx, ny, p = 96, 36, 3
+    cfg, F, obs = _exact_case(nx, ny, M, p, 1, 3e-3)
+    cfg.compat_stale_v = 0
+    half = F[:, :, :, nx // 2:]
+    F[:, :, :, nx // 2:] = half.mean(0) + np.float32(1e-3) * (half - half.mean(0))
+    d_yo = torch.from_numpy(np.stack([obs[k][::p, ::p] for k in (1, 2, 0)]).copy()).cuda()
+    d_in = torch.from_numpy(F).cuda()
+    out = torch.full_like(d_in, float("nan"))
+    mac = torch.full((M, 3, ny, nx), float("nan"), device="cuda")
+    rc, st = _call(cfg, d_in, out, mac, d_yo)
+    assert rc == 0 and st[1] == 0 and st[2] == 0 and st[0] > 1 and nx * ny < st[3] < st[0] * nx * ny, (rc, st)
+    f = out.cpu().numpy().astype(np.float64)
+    rho = f.sum(1)
+    ex, ey = np.arange(9) % 3 - 1, np.arange(9) // 3 - 1
+    c = cfg.u_ref / cfg.cfl
+    got = mac.cpu().numpy()
+    np.testing.assert_allclose(got[:, 0], rho, rtol=1e-6)  # nine roundings of terms up to 1
+    np.testing.assert_allclose(got[:, 1], (f * ex[:, None, None]).sum(1) * c / rho, atol=2e-5)  # the same times c = 20
+    np.testing.assert_allclose(got[:, 2], (f * ey[:, None, None]).sum(1) * c / rho, atol=2e-5)
+    again, mac2 = d_in.clone(), torch.zeros_like(mac)
+    assert _call(cfg, again, again, mac2, d_yo) == (0, st)
+    assert torch.equal(again, out) and torch.equal(mac2, mac)
