@@ -266,10 +266,11 @@ int lbl_event_elapsed(lbl_ctx* ctx, int slot_a, int slot_b, double* ms);
  * host_stats (int[4]: max sweeps, non-converged points, NaN flag, sweep total) is
  * optional; given, the call waits for the stream and returns LBL_ERR_NAN on a NaN
  * in the analysis.  Without it the call does not wait and cannot report a NaN.  Nine or
- * more members are solved without an eigensolver (one sweep per point, never
- * non-converged), but for points whose matrix is ill-conditioned (the observations
- * pull more than about 1e4 times as hard as the inflated background), which the
- * Jacobi iteration solves.
+ * more members are solved without an eigensolver, counted as one sweep per point.
+ * The Jacobi iteration solves the points whose matrix is ill-conditioned (the
+ * observations pull more than about 1e4 times as hard as the inflated background),
+ * and every point when jacobi_tol or jacobi_max_sweeps, which are the iteration's,
+ * are not lbl_config_default's.
  * err (optional) receives a message of at most err_cap bytes. */
 int lbl_letkf_analysis_noalloc(const lbl_config* cfg, const float* f_in, float* f_out, float* mac_out,
                                const float* yo_sites, void* stream, int* host_stats, char* err, size_t err_cap);

@@ -267,6 +267,7 @@ struct AnalysisArgs {
     int nx, ny, M, p, nox, nl_off, nobs;
     float diag, sqrt_m1, tol, c;
     int max_sweeps, write_v;
+    bool iterate;             // the Jacobi iteration for every point (a caller's own tolerance or sweep limit)
     int nl;                   // window half width in sites (n_obs_local)
     double dloc, covinf;      // Gaspari-Cohn length, inflation beta
     int off;                  // window offset (obs_offset)

@@ -1471,8 +1471,9 @@ void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s) {
     obs_table_kernel<<<grid, threads, 0, s>>>(a.f_in, a.yo, a.dY, a.dyo, A, T);
 }
 
+// the direct kernel, the Jacobi kernel for what it leaves, or the Jacobi kernel alone
 void launch_analysis_args(const AnalysisArgs& a, cudaStream_t s) {
-    switch (launch_analysis_direct_args(a, s)) {
+    switch (a.iterate ? Direct::kNone : launch_analysis_direct_args(a, s)) {
         case Direct::kAll: return;
         case Direct::kLeavesSome:  // the points it left, at the iteration's accuracy
             if (a.M <= 16) launch_analysis_args_mp<16>(a, true, s);

@@ -154,6 +154,10 @@ int analysis_noalloc_impl(const lbl_config* cfg, const float* f_in, float* f_out
     a.tol = float(c.jacobi_tol);
     a.c = float(c.u_ref) / float(c.cfl);
     a.max_sweeps = c.jacobi_max_sweeps;
+    // a tolerance or a sweep limit of the caller's own is the iteration's: it then solves every point
+    lbl_config def;
+    lbl_config_default(&def, c.mode, c.nx, M);
+    a.iterate = c.jacobi_tol != def.jacobi_tol || c.jacobi_max_sweeps != def.jacobi_max_sweeps;
     a.write_v = c.compat_stale_v ? 0 : 1;
     a.nl = nl;
     a.dloc = dloc;

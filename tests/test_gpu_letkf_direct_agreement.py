@@ -43,3 +43,26 @@ def test_pointwise_windows(nx, ny, M):
     """Three observations a point, order 8 on sixteen lanes: eight lanes hold no matrix row, and
     their zeros must not reach the reflections."""
     _check(nx, ny, M, 1, 0)
+
+
+@pytest.mark.parametrize("M,p,L", [(9, 1, 0), (16, 4, 1), (32, 2, 0), (32, 4, 1)])
+def test_the_iterations_options_choose_it(M, p, L):
+    """A tolerance or a sweep limit of the caller's own is the Jacobi iteration's: it solves every
+    point, with lbl_assimilate's bits under the same options, and the counters are its own."""
+    cfg, F, obs = _case(64, 32, M, p, L, 1.1, 0.002, 1e-4)
+    cfg.jacobi_tol = 1e-4
+    got, rc, st = _analyse(cfg, F, obs)
+    assert rc == 0 and st[0] > 1 and st[3] > 64 * 32
+    np.testing.assert_array_equal(got, _assimilate(cfg, F, obs))
+    cfg.jacobi_tol, cfg.jacobi_max_sweeps = 1e-6, 1
+    got, rc, st = _analyse(cfg, F, obs)
+    assert rc == 0 and st[0] == 1 and st[1] > 0 and st[3] == 64 * 32
+    np.testing.assert_array_equal(got, _assimilate(cfg, F, obs))
+
+
+@pytest.mark.parametrize("nx,ny,M,p,L", [
+    (64, 32, 9, 4, 1), (64, 32, 16, 4, 1), (64, 32, 17, 4, 1), (64, 32, 32, 4, 1), (64, 32, 16, 2, 0), (96, 36, 32, 2, 0),
+])
+def test_every_form(nx, ny, M, p, L):
+    """The smallest and largest ensembles of both member orders, and the observation space's order 16."""
+    _check(nx, ny, M, p, L)
