@@ -109,6 +109,7 @@ __device__ __forceinline__ float mean_of(float s, float m, float inv_m) {
 constexpr int kB = 10;          // carried rows: nine of R, then g
 constexpr int kMaxPoles = 30;   // shifts of one table
 constexpr int kTables = 20;     // kappa <= 4^1 .. 4^20
+constexpr int kMaxRounds = 6;   // of a CTA
 constexpr float kKappaMax = 1e8f;  // a point of order 16 above it counts as not converged: its mean update is good to 1e-3
 
 // the shifts and weights, one table per kappa = 4^(b+1)
@@ -126,6 +127,7 @@ struct DirParams {
     int nx, ny, nxy, M;
     int p, nsx, nsy, nsites, nobs, nox, nl_off;
     int nbx, nby;           // p x p observation blocks per tile
+    int rounds;             // rounds of points of a CTA (blockIdx.y counts the shares of a tile)
     int ms;                 // floats per slot of the staged window (at least N in the primal form): 4 (mod 8),
                             // so that eight lanes reading 16 bytes of consecutive slots hit different banks
     float inv_sqrt_a, sqrt_beta, c, inv_m;
@@ -351,7 +353,8 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
     }
     __syncthreads();
     const int tw = A.nbx * A.p, npts = tw * A.nby * A.p;
-    const int rounds = (npts + kWarps * S::GPW - 1) / (kWarps * S::GPW);
+    constexpr int kPerRound = kWarps * S::GPW;
+    const int round0 = blockIdx.y * A.rounds, round1 = min(round0 + A.rounds, (npts + kPerRound - 1) / kPerRound);
     // ---- a tile that may hold a point above the limit is left to the Jacobi kernel, before it costs a solve.
     // The trace of C^T C, sum of w |dY|^2 / a, is at least kappa - 1; every member's largest dY of the window
     // and the weights of the pattern (0, 0) bound it to within a factor of a few.
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (!(t * (A.inv_sqrt_a * A.inv_sqrt_a) <= A.limit)) {  // (all warps see the same sum)
 #pragma unroll 1
-            for (int pt = tid; pt < npts; pt += 32 * kWarps) {
+            for (int pt = round0 * kPerRound + tid; pt < min(round1 * kPerRound, npts); pt += 32 * kWarps) {
                 const int i = bx0 * A.p + pt % tw, j = by0 * A.p + pt / tw;
                 if (i < A.nx && j < A.ny) A.mac[i + A.nx * j] = __uint_as_float(kLeftPoint);
             }
@@ -392,7 +395,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
     bool bad = false;
     int noconv = 0;
 #pragma unroll 1
-    for (int round = 0; round < rounds; round++) {
+    for (int round = round0; round < round1; round++) {
         __syncthreads();  // the stages' barriers keep the warps on the same instructions
         const int pt0 = (round * kWarps + warp) * S::GPW;
         // ---- the point; an idle group (a tile's edge) repeats the tile's first point and writes nothing
@@ -950,7 +953,7 @@ __global__ void __launch_bounds__(32 * warps_of(N), N > 16 ? 1 : 2) analysis_dir
     }
     if (bad) atomicOr(A.stats + 2, 1);
     if (noconv) atomicAdd(A.stats + 1, noconv);
-    if (tid == 0) {  // one direct solve per point, counted as one sweep
+    if (tid == 0 && blockIdx.y == 0) {  // one direct solve per point, counted as one sweep
         const int w = max(0, min(tw, A.nx - bx0 * A.p)), h = max(0, min(A.nby * A.p, A.ny - by0 * A.p));
         atomicMax(A.stats + 0, 1);
         atomicAdd(A.stats + 3, w * h);
@@ -1131,9 +1134,17 @@ void launch(const Plan& P, DirParams& A, cudaStream_t s) {
     A.nby = P.nby;
     A.ms = P.ms;
     const int tiles = ((A.nsx + P.nbx - 1) / P.nbx) * ((A.nsy + P.nby - 1) / P.nby);
+    // A tile is at least one block of p x p points, whose rounds follow one another: from p = 9 or 10 on, CTAs of at
+    // most six rounds share it (each stages the window).  With one CTA a tile, an analysis of 64^2 x 16 took 248 us
+    // at p = 16 and 960 at p = 32, where the Jacobi kernel takes 159 and 149 (32 members: 826, 3200; 359, 310).
+    const Variant& V = kVariants[P.variant];
+    const int per_round = warps_of(V.n) * (32 / V.lpp);
+    const int rounds = (P.nbx * A.p * P.nby * A.p + per_round - 1) / per_round;
+    const int shares = (rounds + kMaxRounds - 1) / kMaxRounds;
+    A.rounds = (rounds + shares - 1) / shares;
     PoleTables T = pole_tables();
     void* args[] = {&A, &T};
-    cudaLaunchKernel(kVariants[P.variant].fn, dim3(tiles), dim3(32 * warps_of(kVariants[P.variant].n)), args, P.smem, s);
+    cudaLaunchKernel(V.fn, dim3(tiles, shares), dim3(32 * warps_of(V.n)), args, P.smem, s);
 }
 
 }  // namespace

@@ -1,5 +1,5 @@
 """Edges of the analysis without an eigensolver (csrc/letkf_direct.cu) through the allocation-free
-entry point: windows whose observations weigh nothing, and tiles left to the Jacobi kernel."""
+entry point: windows whose observations weigh nothing, tiles left to the Jacobi kernel, and blocks that several CTAs share."""
 import ctypes
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 
 import lbl
 from test_gpu_letkf_direct import _analyse, _case
+from test_gpu_letkf_direct_agreement import _assimilate
 from test_gpu_letkf_direct_precision import _exact_case
 
 pytestmark = pytest.mark.gpu
@@ -73,3 +74,21 @@ def test_points_left_to_the_iteration(M):
     again, mac2 = d_in.clone(), torch.zeros_like(mac)
     assert _call(cfg, again, again, mac2, d_yo) == (0, st)
     assert torch.equal(again, out) and torch.equal(mac2, mac)
+
+
+@pytest.mark.parametrize("M", [9, 32])
+@pytest.mark.parametrize("nx,ny,p,L", [
+    (64, 20, 4, 1), (96, 32, 8, 1), (288, 18, 9, 1), (160, 20, 10, 0), (64, 64, 16, 1), (64, 64, 64, 1),
+])
+def test_blocks_shared_by_several_ctas(nx, ny, M, p, L):
+    """Blocks of p x p points from one round of a CTA to many: from 9 or 10 on, several CTAs share a
+    block.  Every point is analysed, and counted, once."""
+    cfg, F, obs = _exact_case(nx, ny, M, p, L, 0.3)
+    d_yo = torch.from_numpy(np.stack([obs[k][::p, ::p] for k in (1, 2, 0)]).copy()).cuda()
+    d_in = torch.from_numpy(F).cuda()
+    out = torch.full_like(d_in, float("nan"))
+    rc, st = _call(cfg, d_in, out, torch.zeros((M, 3, ny, nx), device="cuda"), d_yo)
+    assert (rc, st) == (0, [1, 0, 0, nx * ny])
+    want = _assimilate(cfg, F, obs)
+    scale = np.max(np.abs(want - F))
+    assert scale > 1e-4 and np.max(np.abs(out.cpu().numpy() - want)) < 3e-5 * scale + 3 * 2.0 ** -24
