@@ -1075,7 +1075,9 @@ int warp_floats(int v, int mx) {
     }
 }
 
-// the most observations of a point: window slots within the Gaspari-Cohn support (2 d_local)
+// the most observations of a point: window slots within the Gaspari-Cohn support (2 d_local); any number above
+// 16 ends the search, since the observation space is then no choice.  (All p^2 patterns took the host 56 us a
+// call at p = 32, 1 ms at 128; from p = 4 on the first one has more.)
 int max_obs(int p, int nox, int nl_off, int nl, double dloc) {
     if (p == 1) return 3 * nox * nox;
     int best = 0;
@@ -1089,6 +1091,7 @@ int max_obs(int p, int nox, int nl_off, int nl, double dloc) {
                     if (std::sqrt(double(di * di + dj * dj)) / (dloc + 1e-6) <= 2.0) n += 3;
                 }
             best = std::max(best, n);
+            if (best > 16) return best;
         }
     return best;
 }

@@ -1,6 +1,7 @@
 """Edges of the analysis without an eigensolver (csrc/letkf_direct.cu) through the allocation-free
 entry point: windows whose observations weigh nothing, tiles left to the Jacobi kernel, and blocks that several CTAs share."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -92,3 +93,28 @@ def test_blocks_shared_by_several_ctas(nx, ny, M, p, L):
     want = _assimilate(cfg, F, obs)
     scale = np.max(np.abs(want - F))
     assert scale > 1e-4 and np.max(np.abs(out.cpu().numpy() - want)) < 3e-5 * scale + 3 * 2.0 ** -24
+
+
+def test_host_cost_does_not_grow_with_the_block():
+    """Choosing the form takes a few window patterns, not all p^2 of them: a call at p = 64 costs the
+    host about what one at p = 4 does (13 us; with all patterns 195).  Best of many, and a
+    factor of three for the difference."""
+    best = {}
+    for p in (4, 64):
+        cfg = lbl.config_default("DA_LETKF", 128, 16, ny=128, da_xyprune=p, letkf_rloc_len=1)
+        d_in = torch.ones((16, 9, 128, 128), device="cuda") / 9
+        out, mac = torch.empty_like(d_in), torch.empty((16, 3, 128, 128), device="cuda")
+        yo = torch.zeros((3, 128 // p, 128 // p), device="cuda")
+        fn, stream = lbl.load_library().lbl_letkf_analysis_noalloc, torch.cuda.current_stream().cuda_stream
+        times = []
+        for _ in range(60):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            rc = fn(ctypes.byref(cfg), d_in.data_ptr(), out.data_ptr(), mac.data_ptr(), yo.data_ptr(), stream, None,
+                    None, 0)
+            times.append(time.perf_counter() - t0)
+            assert rc == 0
+        torch.cuda.synchronize()
+        best[p] = min(times)
+    print({p: f"{t * 1e6:.1f} us" for p, t in best.items()})
+    assert best[64] < 3 * best[4]
