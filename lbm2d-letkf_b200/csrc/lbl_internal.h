@@ -273,6 +273,7 @@ struct AnalysisArgs {
     int off;                  // window offset (obs_offset)
     double sig_u, sig_rho;    // observation errors
 };
+int analysis_args_prepare();  // once per device, before any capture
 // the observation operator, the weight table a.wtab and the cleared counters a.stats, in one launch
 void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s);
 // ---- the Gram on the tcgen05 tensor cores (gram_tc.cu) ----

@@ -989,7 +989,7 @@ struct Agm {
 
 // t^-1/2 = D prod(t + c_2l) / prod(t + c_2l-1) on [1, kappa], c_l = (sn/cn)^2(l K / 2N) for
 // m = 1 - 1/kappa (Zolotarev 1877), in partial fractions; D levels the relative error's two
-// extremes, which it takes at t = 1 and at its other alternation points.  Returns the error.
+// extremes, sampled at 16 points for each of its 2 N + 1 alternations.  Returns the error.
 double zolotarev(double kappa, int N, double* s, double* w) {
     const Agm g(1.0 / kappa);
     const double K = g.K();
@@ -1005,8 +1005,10 @@ double zolotarev(double kappa, int N, double* s, double* w) {
         w[i] = v;
     }
     double lo = 1e300, hi = -1e300;
-    for (int e = 0; e <= 4000; e++) {
-        const double t = std::exp(std::log(kappa) * e / 4000.0);
+    const int samples = 16 * (2 * N + 1);
+    const double step = std::pow(kappa, 1.0 / samples);
+    double t = 1.0;
+    for (int e = 0; e <= samples; e++, t *= step) {
         double f = 0;
         for (int i = 0; i < N; i++) f += w[i] / (t + s[i]);
         f *= std::sqrt(t);
@@ -1021,11 +1023,10 @@ const PoleTables& pole_tables() {
     static const PoleTables tables = [] {
         PoleTables T{};
         double kappa = 4.0;
+        int n = 3;
         for (int b = 0; b < kTables; b++, kappa *= 4.0) {
             double s[kMaxPoles], w[kMaxPoles];
-            int n = 3;
-            while (n < kMaxPoles && zolotarev(kappa, n, s, w) > 2e-8) n++;
-            zolotarev(kappa, n, s, w);
+            while (zolotarev(kappa, n, s, w) > 2e-8 && n < kMaxPoles) n++;  // (a wider spectrum takes no fewer)
             T.n[b] = n;
             for (int i = 0; i < n; i++) {
                 T.s[b][i] = float(s[i]);

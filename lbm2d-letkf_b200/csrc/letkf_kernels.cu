@@ -1330,19 +1330,27 @@ size_t analysis_smem_bytes(int M, int nobs) {
 // opt in to large dynamic shared memory once per device (not allowed during capture)
 int analysis_prepare() {
     const int lim = 200 * 1024;
-    int rc = direct_prepare();
+    int rc = 0;
     rc |= int(cudaFuncSetAttribute(analysis_kernel<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-    rc |= int(cudaFuncSetAttribute(analysis_left_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
-    rc |= int(cudaFuncSetAttribute(analysis_left_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     rc |= int(cudaFuncSetAttribute(analysis_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    return rc;
+}
+
+// the same for the kernels that only the allocation-free entry point launches, and the direct solver's tables: not
+// part of lbl_create, which they made 14 ms longer
+int analysis_args_prepare() {
+    const int lim = 200 * 1024;
+    int rc = analysis_prepare() | direct_prepare();
+    rc |= int(cudaFuncSetAttribute(analysis_left_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    rc |= int(cudaFuncSetAttribute(analysis_left_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
     return rc;
 }
 

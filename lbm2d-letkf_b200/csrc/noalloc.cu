@@ -64,7 +64,7 @@ int scratch_for_current_device(float** out) {
         e = cudaGetSymbolAddress(reinterpret_cast<void**>(&ptr), g_noalloc_scratch);
         if (e != cudaSuccess || !ptr)
             return noalloc_fail(LBL_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-        if (lbl::analysis_prepare() != 0) return noalloc_fail(LBL_ERR_CUDA, "cudaFuncSetAttribute(analysis_kernel) failed");
+        if (lbl::analysis_args_prepare() != 0) return noalloc_fail(LBL_ERR_CUDA, "cudaFuncSetAttribute(analysis_kernel) failed");
         g_scratch_addr[dev] = ptr;
     }
     *out = g_scratch_addr[dev];
