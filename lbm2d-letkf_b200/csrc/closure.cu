@@ -468,7 +468,7 @@ int lbl_set_closure(lbl_ctx* ctx, const float* params, double nu_ref, double dx_
         ctx->err = "cudaMalloc(closure parameters) failed";
         return LBL_ERR_CUDA;
     }
-    if (cudaMemcpy(ctx->d_closure, pack.data(), sizeof(uint32_t) * kPackWords, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (upload(ctx->d_closure, pack.data(), sizeof(uint32_t) * kPackWords, ctx->stream) != cudaSuccess)
         return LBL_ERR_CUDA;
     ctx->closure_sc.dx = ctx->P.dx;
     ctx->closure_sc.nu_ref = nu_ref > 0 ? float(nu_ref) : ctx->P.nu;

@@ -372,7 +372,7 @@ int check_timeout(lbl_ctx* ctx) {
     int h = 0;
     LBL_CK(cudaMemcpy(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (h) {
-        cudaMemset(ctx->d_err, 0, sizeof(int));
+        cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream);
         return fail(ctx, LBL_ERR_TIMEOUT, std::string(h == 4 ? "tensor-core Gram: the MMA completion wait"
                                                                : "stream-collide: a bounded shared-memory pipeline wait") +
                                               " gave up (code " + std::to_string(h) + ")");
@@ -430,7 +430,7 @@ int ic_member(lbl_ctx* ctx, int seed, std::vector<float>& u, std::vector<float>&
     const size_t nxy = size_t(nx) * ny;
     LBL_CK(cudaMalloc(&d_tab, sizeof(double) * std::max<size_t>(tab.size(), 1)));
     LBL_CK(cudaMalloc(&d_uv, sizeof(float) * 2 * nxy));
-    LBL_CK(cudaMemcpy(d_tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+    LBL_CK(upload(d_tab, tab.data(), sizeof(double) * tab.size(), ctx->stream));
     launch_ic_velocity(d_tab, n, nx, ny, d_uv, d_uv + nxy, ctx->stream);
     LBL_CK(cudaGetLastError());
     u.resize(nxy); v.resize(nxy);
@@ -498,7 +498,7 @@ int build_weight_table(lbl_ctx* ctx) {
             cnt[pat] = n;
         }
     LBL_CK(cudaMalloc(&ctx->d_wtab, sizeof(int) * tab.size()));
-    LBL_CK(cudaMemcpy(ctx->d_wtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice));
+    LBL_CK(upload(ctx->d_wtab, tab.data(), sizeof(int) * tab.size(), ctx->stream));
     if (cfg.gram == LBL_GRAM_TF32X3) {  // the same weights, dense per pattern, for the tensor-core Gram
         const int kpad = (G.nobs + 7) & ~7;
         std::vector<float> dense(size_t(np) * kpad, 0.f);
@@ -508,7 +508,7 @@ int build_weight_table(lbl_ctx* ctx) {
                 std::memcpy(&dense[size_t(pat) * kpad + e[0]], &e[3], sizeof(float));
             }
         LBL_CK(cudaMalloc(&ctx->d_wdense, sizeof(float) * dense.size()));
-        LBL_CK(cudaMemcpy(ctx->d_wdense, dense.data(), sizeof(float) * dense.size(), cudaMemcpyHostToDevice));
+        LBL_CK(upload(ctx->d_wdense, dense.data(), sizeof(float) * dense.size(), ctx->stream));
         const int mpq = gram_tc_mp(ctx->P.M);
         LBL_CK(cudaMalloc(&ctx->d_Q, sizeof(float) * size_t(ctx->P.nxy) * (size_t(mpq) * mpq + mpq)));
         if (gram_tc_prepare() != 0) return fail(ctx, LBL_ERR_CUDA, "cudaFuncSetAttribute(gram_tc_kernel) failed");
@@ -575,7 +575,7 @@ int create_impl(const lbl_config* cfg, int device, lbl_ctx* ctx) {
             LBL_CK(cudaMalloc(&ctx->f[b], sizeof(float) * M * kQ * nxy));
         }
         LBL_CK(cudaMalloc(&ctx->mac[b], sizeof(float) * M * 3 * nxy));
-        LBL_CK(cudaMemset(ctx->mac[b], 0, sizeof(float) * M * 3 * nxy));
+        LBL_CK(cudaMemsetAsync(ctx->mac[b], 0, sizeof(float) * M * 3 * nxy, ctx->stream));
     }
     // forcing mode table (data.cu:161-237), amplitudes normalised in long double
     {
@@ -609,9 +609,9 @@ int create_impl(const lbl_config* cfg, int device, lbl_ctx* ctx) {
             amps[n + i] = double(ctx->h_amp[i] * 2) * M_PI * double(-ctx->h_kx[i]);
         }
         LBL_CK(cudaMalloc(&ctx->d_modes, sizeof(float) * 2 * n));
-        LBL_CK(cudaMemcpy(ctx->d_modes, tab.data(), sizeof(float) * 2 * n, cudaMemcpyHostToDevice));
+        LBL_CK(upload(ctx->d_modes, tab.data(), sizeof(float) * 2 * n, ctx->stream));
         LBL_CK(cudaMalloc(&ctx->d_amps, sizeof(double) * 2 * n));
-        LBL_CK(cudaMemcpy(ctx->d_amps, amps.data(), sizeof(double) * 2 * n, cudaMemcpyHostToDevice));
+        LBL_CK(upload(ctx->d_amps, amps.data(), sizeof(double) * 2 * n, ctx->stream));
         std::copy(amps.begin(), amps.end(), ctx->h_amps);
         ctx->n_rand_buf = n * 4096;                                        // data.cu:297
         LBL_CK(cudaMalloc(&ctx->d_pool, sizeof(float) * ctx->pool_slots * size_t(ctx->n_rand_buf)));
@@ -619,7 +619,7 @@ int create_impl(const lbl_config* cfg, int device, lbl_ctx* ctx) {
     // steps of forcing one graph can hold: 256 MB of fields (512 steps at 256^2, 128 at 512^2)
     ctx->force_cap = int(std::max<long long>(8, std::min<long long>(1023, (256ll << 20) / (8ll * nxy))));
     LBL_CK(cudaMalloc(&ctx->d_force, sizeof(float) * 2 * nxy * ctx->force_cap));
-    LBL_CK(cudaMemset(ctx->d_force, 0, sizeof(float) * 2 * nxy * ctx->force_cap));
+    LBL_CK(cudaMemsetAsync(ctx->d_force, 0, sizeof(float) * 2 * nxy * ctx->force_cap, ctx->stream));
     LBL_CK(cudaMalloc(&ctx->d_sched, sizeof(int) * ctx->force_cap));
     for (int b = 0; b < 2; b++) LBL_CK(cudaMallocHost(&ctx->h_sched[b], sizeof(int) * ctx->force_cap));
     LBL_CKR(curandCreateGenerator(&ctx->gen, CURAND_RNG_PSEUDO_MTGP32));   // data.cu:293-294
@@ -638,12 +638,12 @@ int create_impl(const lbl_config* cfg, int device, lbl_ctx* ctx) {
         LBL_CK(cudaMalloc(&ctx->d_dyo, sizeof(float) * 3 * ns));
     }
     LBL_CK(cudaMalloc(&ctx->d_stats, sizeof(int) * 4));
-    LBL_CK(cudaMemset(ctx->d_stats, 0, sizeof(int) * 4));  // max sweeps, non-converged, NaN, sweep total
+    LBL_CK(cudaMemsetAsync(ctx->d_stats, 0, sizeof(int) * 4, ctx->stream));  // max sweeps, non-converged, NaN, sweep total
     LBL_CK(cudaMalloc(&ctx->d_red, sizeof(double) * 8));
     LBL_CK(cudaMalloc(&ctx->d_tmp, sizeof(float) * 6 * nxy));
     ctx->d_acc = ctx->d_tmp + 2 * nxy;
     LBL_CK(cudaMalloc(&ctx->d_err, sizeof(int)));
-    LBL_CK(cudaMemset(ctx->d_err, 0, sizeof(int)));
+    LBL_CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     if (cfg->lbm_variant == LBL_LBM_TMA && !ctx->f16 && lbm_tma_supported(cfg->nx)) {
         ctx->use_tma = make_population_map(ctx, ctx->f[0], &ctx->tmap[0]) &&
                        make_population_map(ctx, ctx->f[1], &ctx->tmap[1]) && lbm_tma_prepare(cfg->nx) == 0;
@@ -709,16 +709,17 @@ void destroy_impl(lbl_ctx* ctx) {
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
 }
 
-// one member's FP32 populations [9][ny][nx] to/from buffer b, converting for FP16 storage
+// one member's FP32 populations [9][ny][nx] to/from buffer b, converting for FP16 storage; the caller waits for the
+// upload before f goes
 int upload_member(lbl_ctx* ctx, int b, int m, const float* f) {
     const size_t n = size_t(kQ) * ctx->P.nxy;
     if (!ctx->f16) {
-        LBL_CK(cudaMemcpy(ctx->f[b] + size_t(m) * n, f, sizeof(float) * n, cudaMemcpyHostToDevice));
+        LBL_CK(cudaMemcpyAsync(ctx->f[b] + size_t(m) * n, f, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
         return LBL_OK;
     }
     std::vector<__half> h(n);
     for (size_t e = 0; e < n; e++) h[e] = __float2half_rn(f[e] - wq_h(int(e / ctx->P.nxy)));
-    LBL_CK(cudaMemcpy(ctx->h[b] + size_t(m) * n, h.data(), sizeof(__half) * n, cudaMemcpyHostToDevice));
+    LBL_CK(upload(ctx->h[b] + size_t(m) * n, h.data(), sizeof(__half) * n, ctx->stream));
     return LBL_OK;
 }
 
@@ -758,9 +759,10 @@ int init_impl(lbl_ctx* ctx, int ens_offset) {
         }
         for (int b = 0; b < 2; b++) {  // data_0_ and data_1_ both start from the IC (data.h:55)
             LBL_TRY(upload_member(ctx, b, m, fh.data()));
-            LBL_CK(cudaMemcpy(ctx->mac[b] + size_t(m) * 3 * nxy, mh.data(), sizeof(float) * 3 * nxy,
-                              cudaMemcpyHostToDevice));
+            LBL_CK(cudaMemcpyAsync(ctx->mac[b] + size_t(m) * 3 * nxy, mh.data(), sizeof(float) * 3 * nxy,
+                                   cudaMemcpyHostToDevice, ctx->stream));
         }
+        LBL_CK(cudaStreamSynchronize(ctx->stream));
     }
     // forcing: cursor starts "outdated", two update_forces calls at init (data.cu:236, :158)
     ctx->fc_free_recorded = false;
@@ -1748,7 +1750,7 @@ int batch_table(lbl_batch* b, int cur_mask, BatchExp** out) {
         for (size_t e = 0; e < t.size(); e++) t[e].cur = (cur_mask >> e) & 1;
         BatchExp* d = nullptr;
         BATCH_CK(cudaMalloc(&d, sizeof(BatchExp) * t.size()));
-        BATCH_CK(cudaMemcpy(d, t.data(), sizeof(BatchExp) * t.size(), cudaMemcpyHostToDevice));
+        BATCH_CK(upload(d, t.data(), sizeof(BatchExp) * t.size(), b->stream));
         it = b->tables.emplace(cur_mask, d).first;
     }
     *out = it->second;

@@ -183,6 +183,15 @@ struct lbl_ctx {
 
 namespace lbl {
 
+// Host memory to the device, done when it returns.  On the stream whose kernels read it: the contexts' streams do not
+// wait for the legacy stream, and cudaMemcpy from pageable memory may return with the copy still under way
+// there, held up by whatever shares its hardware queue; a batch's first step could then read its table of
+// pointers before it has arrived.
+inline cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+}
+
 // ---- kernels (lbm_kernels.cu, compiled with the reference's -use_fast_math) ----
 void launch_ic_velocity(const double* modes /*[4][n]*/, int n_modes, int nx, int ny,
                         float* u, float* v, cudaStream_t s);
