@@ -279,7 +279,6 @@ struct AnalysisArgs {
     bool iterate;             // the Jacobi iteration for every point (a caller's own tolerance or sweep limit)
     int nl;                   // window half width in sites (n_obs_local)
     double dloc, covinf;      // Gaspari-Cohn length, inflation beta
-    int off;                  // window offset (obs_offset)
     double sig_u, sig_rho;    // observation errors
 };
 int analysis_args_prepare();  // once per device, before any capture

@@ -1,7 +1,8 @@
 // letkf_direct.cu -- the LETKF local analysis without an eigensolver, for sm_100a: the solver of
 // the allocation-free entry point (noalloc.cu), 9 to 32 members.  The contexts' analyses keep the Jacobi
 // kernels (letkf_kernels.cu): a run of cycles amplifies last-bit differences, and theirs must go on
-// reproducing earlier runs; the two solvers agree to about 1e-5 of an increment, each that far from FP64.
+// reproducing earlier runs; the two solvers' analyses agree to half an ulp of a population (2e-5 of an
+// increment of 1.5e-3).
 //
 // The analysis applies W = sqrt(M-1) Q^-1/2 + Q^-1 c 1^T, Q = (M-1)/beta I + dY^T R^-1 dY
 // (letkf_solver.h:243-316), to nine rows dX only, so the eigenvectors of Q are never needed.
@@ -146,8 +147,9 @@ struct Shape {
 };
 // Warps of a CTA.  The kernel's code is larger than the instruction caches near the schedulers, so an
 // SM's warps walk it together: one CTA of twelve warps (168 registers) per SM above order 16, two of
-// eight (128 registers) below, with a barrier between the stages of a point.  Independent CTAs of
-// four warps spent half of their cycles waiting for instructions.
+// eight (128 registers) below (one where shared memory holds no second: the dual order 16 from 21 members
+// on, 117 kB), with a barrier between the stages of a point.  Independent CTAs of four warps spent half of
+// their cycles waiting for instructions.
 __host__ __device__ constexpr int warps_of(int n) { return n > 16 ? 12 : 8; }
 // floats of a point's shared region; mx = members rounded up to 4.  Dual: dX as [member][12], then the point's
 // weighted window [member][N]; primal: the rows on their way in, [12][N]
@@ -1105,11 +1107,12 @@ struct Plan {
 Plan make_plan(int M, int p, int nox, int nl_off, int nl, double dloc, int nsx, int nsy) {
     Plan P;
     const int obs = max_obs(p, nox, nl_off, nl, dloc), nobs = 3 * nox * nox;
-    // The smaller of the two spaces.  An analysis of 128^2 points, this kernel against the Jacobi kernel
-    // (us, both with the observation operator): pointwise (3 observations) M = 4: 70 / 51, 8: 72 / 80, 16: 87 / 157,
-    // 32: 121 / 718; DA_XYPRUNE 2 (12) M = 4: 59 / 57, 8: 68 / 86, 16: 103 / 178; DA_XYPRUNE 4, LETKF_RLOC_LEN 1
-    // (42) M = 6: 82 / 87, 8: 87 / 86, 12: 97 / 174, 24: 392 / 918; 256^2 x 16: 367 / 474, 256^2 x 32: 1699 / 2380.
-    // Up to 8 members, where the Jacobi kernel packs four or eight points into a warp, it stays.
+    // The smaller of the two spaces.  A call of the entry point, this way / all by the Jacobi kernel (us): pointwise (3
+    // observations) at 128^2, 9 members 73 / 134, 16: 79 / 137, 17: 93 / 603, 32: 114 / 667; DA_XYPRUNE 2 (15) at 160 x 96,
+    // 16: 95 / 173, 17: 103 / 689, 32: 159 / 776; DA_XYPRUNE 4, LETKF_RLOC_LEN 1 (42) at 256^2, 9: 289 / 420, 16: 353 / 467,
+    // 17: 1071 / 2217, 32: 1658 / 2388.
+    // Up to 8 members the gain was small (pointwise at 128^2, 4 members 70 / 51, 8: 72 / 80), and the entry point keeps
+    // lbl_assimilate's analysis to the bit, within the 1e-7 that its velocities are held to there.
     if (M <= 8 || M > 32) return P;
     int v = 1;
     if (obs <= 16 && obs < M) v = obs <= 8 ? 2 : 3;
@@ -1127,7 +1130,7 @@ Plan make_plan(int M, int p, int nox, int nl_off, int nl, double dloc, int nsx, 
         if (P.smem <= kAnalysisSmemLimit) break;
         if (P.nbx > 1) P.nbx /= 2;
         else if (P.nby > 1) P.nby /= 2;
-        else return P;  // the window alone is too large
+        else return P;  // the window alone is too large (none that the entry point accepts: 187 kB at most)
     }
     P.variant = v;
     return P;

@@ -147,7 +147,7 @@ __device__ double gc_weight_rn(double d) {
 // operator: a call at 128^2 x 4 pointwise 46 against 43 us now, at 160 x 96 x 23 every 2 points 162 / 141, at
 // 256^2 x 16 every 4 points 382 / 352.)
 struct TableJob {
-    int obs_blocks, nl, off;
+    int obs_blocks, nl;
     double dloc, sig_u, sig_rho;
     int *tab, *stats;
 };
@@ -1474,7 +1474,7 @@ void launch_obs_ensemble_args(const AnalysisArgs& a, cudaStream_t s) {
     const AnaParams A = params_from_args(a);
     const int threads = 256;
     const long long total = (long long)A.nsites * 32;
-    TableJob T{int((total + threads - 1) / threads), a.nl, a.off, a.dloc, a.sig_u, a.sig_rho, a.wtab, a.stats};
+    TableJob T{int((total + threads - 1) / threads), a.nl, a.dloc, a.sig_u, a.sig_rho, a.wtab, a.stats};
     const int grid = T.obs_blocks + (a.p * a.p * 32 + threads - 1) / threads;
     obs_table_kernel<<<grid, threads, 0, s>>>(a.f_in, a.yo, a.dY, a.dyo, A, T);
 }

@@ -162,7 +162,6 @@ int analysis_noalloc_impl(const lbl_config* cfg, const float* f_in, float* f_out
     a.nl = nl;
     a.dloc = dloc;
     a.covinf = c.letkf_covinf;
-    a.off = off;
     a.sig_u = c.obs_error_u;
     a.sig_rho = c.obs_error_rho;
     lbl::launch_obs_ensemble_args(a, s);
