@@ -272,7 +272,8 @@ struct AnalysisArgs {
     float* dY;                // [3][nsites][M] scratch
     float* dyo;               // [3][nsites] scratch
     int* wtab;                // int4 [p*p][nobs] + int [p*p] counts, rebuilt by launch_obs_ensemble_args
-    int* stats;               // int[5] scratch: the four counters, then 1 when the direct solver left a point
+    int* stats;               // int[9] scratch: the four counters, 1 when the direct solver left a point, the
+                              // weights of the three variables, the left points' work counter
     int nx, ny, M, p, nox, nl_off, nobs;
     float diag, sqrt_m1, tol, c;
     int max_sweeps, write_v;

@@ -995,7 +995,7 @@ struct Agm {
 double zolotarev(double kappa, int N, double* s, double* w) {
     const Agm g(1.0 / kappa);
     const double K = g.K();
-    std::vector<double> c(2 * N);
+    double c[2 * kMaxPoles];  // (no allocation: the entry point is C's)
     for (int l = 1; l < 2 * N; l++) {
         const double t = g.tan_am(l * K / (2.0 * N));
         c[l] = t * t;
@@ -1057,7 +1057,7 @@ const Variant kVariants[] = {
 // Jacobi kernel.  Rms error against FP64, of an increment, this kernel / the Jacobi kernel (64 x 32 points, an exact
 // operator, by the largest trace):
 //   primal  1e3: 16 members 1.3e-7 / 3.5e-7, 32 1.1e-7 / 5.6e-7; 1.4e4 (27 observations): 16 members 3.8e-7 / 3.2e-7,
-//           32 1.4e-6 / 1.3e-6; 1.5e6: 6.0e-7 / 3.8e-7, 7.3e-5 / 2.9e-5; 1.5e8: 24 members 2.6e-1 / 1.2e-2
+//           32 1.4e-6 / 1.3e-6; 1.5e6: 6.0e-7 / 3.8e-7, 7.3e-5 / 2.9e-5; 1.5e7: 6.2e-7 / 3.7e-7, 1.2e-4 / 4.6e-5
 //   dual    order 16, 32 members: 1e3 1.4e-8 / 2.9e-7, 1.6e5 1e-7 / 3.9e-4, 1e7 5e-6 / 5e-3, 1.6e8 2e-4 / 0.14, 6e8 5e-3 /
 //           2e4 (not converged); order 8: 1.8e-8 up to 6e11: no limit
 // The reduction keeps an eigenvalue to 2^-24 of the largest; in the member space, one of every window's is the
