@@ -213,8 +213,8 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 }
 
 // Two FP32 multiply-adds (multiplies), PK: in one instruction (sm_100).  Each half rounds as the scalar
-// one, so sums kept in even and odd halves and element-wise updates keep their bits.  The analysis phase,
-// packed against scalar: 512^2 x 64 (the wide kernel) 44.7 / 47.8 ms, 256^2 x 64 13.9 / 15.0, 256^2 x 32 2.27 / 2.33 ms,
+// one, so sums kept in even and odd halves and element-wise updates keep their bits.  The first analysis
+// of a fresh ensemble, packed against scalar: 512^2 x 64 (the wide kernel) 44.7 / 47.8 ms (in cycles 52.3 / 57.1), 256^2 x 64 13.9 / 15.0, 256^2 x 32 2.27 / 2.33 ms,
 // 160 x 96 x 23 0.78 / 0.81; but 256^2 x 16 0.49 / 0.47 and 64^2 x 8 0.107 / 0.088 ms, where the columns are short
 // and every element also passes through a shuffle: those stay scalar.
 template <bool PK>
