@@ -165,12 +165,26 @@ __global__ void __launch_bounds__(256) member_fields_kernel(const float* __restr
 
 }  // namespace
 
-void launch_ens_stats(const lbl_ctx* c, const float* mac, float* stats, cudaStream_t s) {
-    ens_stats_kernel<<<(c->P.nxy + 255) / 256, 256, 0, s>>>(mac, c->P.nx, c->P.ny, c->P.M, c->P.two_dx, stats);
+// The accessors' launches return their own status: the thread's last error may be an earlier call's, such as
+// a context asked for on a device that is not there.
+namespace {
+cudaLaunchConfig_t per_cell(const lbl_ctx* c, cudaStream_t s) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((c->P.nxy + 255) / 256);
+    lc.blockDim = dim3(256);
+    lc.stream = s;
+    return lc;
+}
+}  // namespace
+
+cudaError_t launch_ens_stats(const lbl_ctx* c, const float* mac, float* stats, cudaStream_t s) {
+    const cudaLaunchConfig_t lc = per_cell(c, s);
+    return cudaLaunchKernelEx(&lc, ens_stats_kernel, mac, c->P.nx, c->P.ny, c->P.M, c->P.two_dx, stats);
 }
 
-void launch_member_fields(const lbl_ctx* c, const float* mac, float* out, cudaStream_t s) {
-    member_fields_kernel<<<(c->P.nxy + 255) / 256, 256, 0, s>>>(mac, c->P.nx, c->P.ny, c->P.two_dx, out);
+cudaError_t launch_member_fields(const lbl_ctx* c, const float* mac, float* out, cudaStream_t s) {
+    const cudaLaunchConfig_t lc = per_cell(c, s);
+    return cudaLaunchKernelEx(&lc, member_fields_kernel, mac, c->P.nx, c->P.ny, c->P.two_dx, out);
 }
 
 void launch_output_fields(const lbl_ctx* c, const float* mac, float* vor, float* stats, int* nan, cudaStream_t s) {

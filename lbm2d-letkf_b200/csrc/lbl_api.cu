@@ -975,7 +975,6 @@ int write_output_files(lbl_ctx* ctx, int t, const std::string& pre, std::string&
 int read_accessor(lbl_ctx* ctx, float* const (&out)[4]) {
     const size_t nxy = size_t(ctx->P.nxy), bytes = sizeof(float) * nxy;
     const bool one = bytes <= 128 * 1024;
-    LBL_CK(cudaGetLastError());
     if (one) {
         ctx->h_acc.resize(4 * nxy);
         LBL_CK(cudaMemcpyAsync(ctx->h_acc.data(), ctx->d_acc, 4 * bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1256,7 +1255,7 @@ int lbl_set_f(lbl_ctx* ctx, int member, const float* f) {
 int lbl_get_fields(lbl_ctx* ctx, int member, float* rho, float* u, float* v, float* vor) {
     if (!ctx || member < 0 || member >= ctx->P.M) return LBL_ERR_ARG;
     LBL_TRY(set_device(ctx));
-    launch_member_fields(ctx, ctx->mac[ctx->cur] + size_t(member) * 3 * ctx->P.nxy, ctx->d_acc, ctx->stream);
+    LBL_CK(launch_member_fields(ctx, ctx->mac[ctx->cur] + size_t(member) * 3 * ctx->P.nxy, ctx->d_acc, ctx->stream));
     float* out[4] = {rho, u, v, vor};
     return read_accessor(ctx, out);
 }
@@ -1264,7 +1263,7 @@ int lbl_get_fields(lbl_ctx* ctx, int member, float* rho, float* u, float* v, flo
 int lbl_get_ens_stats(lbl_ctx* ctx, float* u_mean, float* v_mean, float* vor_mean, float* vor_std) {
     if (!ctx) return LBL_ERR_ARG;
     LBL_TRY(set_device(ctx));
-    launch_ens_stats(ctx, ctx->mac[ctx->cur], ctx->d_acc, ctx->stream);
+    LBL_CK(launch_ens_stats(ctx, ctx->mac[ctx->cur], ctx->d_acc, ctx->stream));
     float* out[4] = {u_mean, v_mean, vor_mean, vor_std};
     return read_accessor(ctx, out);
 }

@@ -318,8 +318,8 @@ void launch_diag(const lbl_ctx* c, const float* mac, int member, double* red, cu
 // mean vor, std vor) in the reference's FP32 order; *nan |= 1 on a NaN vorticity
 void launch_output_fields(const lbl_ctx* c, const float* mac, float* vor, float* stats, int* nan, cudaStream_t s);
 // the statistics alone, and one member's rho, u, v and vorticity, [4][nxy], for the accessors
-void launch_ens_stats(const lbl_ctx* c, const float* mac, float* stats, cudaStream_t s);
-void launch_member_fields(const lbl_ctx* c, const float* mac, float* out, cudaStream_t s);
+cudaError_t launch_ens_stats(const lbl_ctx* c, const float* mac, float* stats, cudaStream_t s);
+cudaError_t launch_member_fields(const lbl_ctx* c, const float* mac, float* out, cudaStream_t s);
 void launch_rmse(const lbl_ctx* c, const float* mac, const float* ut, const float* vt, double* red,
                  cudaStream_t s);
 void launch_rmse_finish(const lbl_ctx* c, double* red, cudaStream_t s);

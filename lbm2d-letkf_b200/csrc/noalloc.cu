@@ -120,6 +120,7 @@ int analysis_noalloc_impl(const lbl_config* cfg, const float* f_in, float* f_out
     const int nobs = 3 * nox * nox;
     const int M = c.n_ens;
     const size_t nsites = size_t(c.nx / p) * (c.ny / p);
+    // (the Jacobi kernel's window, since it may be given any point)
     if (lbl::analysis_smem_bytes(M, nobs) > lbl::kAnalysisSmemLimit)
         return noalloc_fail(LBL_ERR_UNSUPPORTED, "observation window too large for the analysis kernel");
 
